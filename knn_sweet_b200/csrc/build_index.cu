@@ -168,39 +168,34 @@ __global__ void rep_pick_kernel(const float4 *__restrict__ rows, int dp4,
 // here they are computed directly, which cannot go negative.
 // Representatives are staged through shared memory in tiles.
 // ---------------------------------------------------------------------------
+constexpr int kAssignPoints = 2;  // points per thread
+
 template <int DP4>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
     assign_kernel(const float4 *__restrict__ rows, int64_t n,
                   const float4 *__restrict__ reps, int R,
                   int32_t *__restrict__ cl, float *__restrict__ dr) {
   constexpr int TILE = (DP4 <= 2) ? 1024 : (DP4 <= 4 ? 512 : 256);
-  __shared__ float4 srep[TILE * DP4];
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  float4 p[DP4];
+  __shared__ __align__(16) float srep[TILE * DP4 * 4];
+  const int64_t i0 = blockIdx.x * (int64_t)(128 * kAssignPoints) + threadIdx.x;
+  NearestRep<DP4, kAssignPoints> nr;
 #pragma unroll
-  for (int c = 0; c < DP4; c++)
-    p[c] = i < n ? rows[i * DP4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
-  // bi starts at 0 so that a point with a NaN coordinate (no comparison
-  // succeeds) still lands in a valid cluster.
-  float best = __int_as_float(0x7f7fffff);  // FLT_MAX
-  int bi = 0;
+  for (int t = 0; t < kAssignPoints; t++)
+    nr.load(t, i0 + 128 * t < n ? rows + (i0 + 128 * t) * DP4 : nullptr);
   for (int base = 0; base < R; base += TILE) {
-    int cnt = min(TILE, R - base);
+    const int cnt = min(TILE, R - base);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * DP4; t += blockDim.x)
-      srep[t] = reps[(int64_t)base * DP4 + t];
+    stage_reps<DP4>(reps + (int64_t)base * DP4, cnt, srep, TILE);
     __syncthreads();
-    for (int j = 0; j < cnt; j++) {
-      float v = dist2_rows<DP4>(p, srep + j * DP4);
-      if (v < best) {
-        best = v;
-        bi = base + j;
-      }
-    }
+    nr.scan(srep, TILE, cnt, base);
   }
-  if (i < n) {
-    cl[i] = bi;
-    dr[i] = sqrtf(best);
+#pragma unroll
+  for (int t = 0; t < kAssignPoints; t++) {
+    const int64_t i = i0 + 128 * t;
+    if (i < n) {
+      cl[i] = nearest_of_quad<DP4>(rows + i * DP4, reps, R, nr.quad[t], nr.best[t]);
+      dr[i] = sqrtf(nr.best[t]);
+    }
   }
 }
 
@@ -666,11 +661,11 @@ int launch_rep_select(const float4 *rows, int dp4, const int32_t *cand_dev,
 int launch_assign(const float4 *rows, int64_t n, int dp4, const float4 *reps,
                   int R, int32_t *cl, float *dr, cudaStream_t s) {
   if (n == 0) return KNN_OK;
-  int blocks = (int)((n + 255) / 256);
+  const int blocks = (int)((n + 255) / 256);  // 256 points each, in both kernels
   switch (dp4) {
 #define KNN_ASSIGN_CASE(D)                                                   \
   case D:                                                                    \
-    assign_kernel<D><<<blocks, 256, 0, s>>>(rows, n, reps, R, cl, dr);       \
+    assign_kernel<D><<<blocks, 128, 0, s>>>(rows, n, reps, R, cl, dr);       \
     break;
     KNN_ASSIGN_CASE(1)
     KNN_ASSIGN_CASE(2)

@@ -116,6 +116,104 @@ __device__ __forceinline__ float dist2_rows_rt(const float4 *__restrict__ a,
   return acc;
 }
 
+// ---------------------------------------------------------------------------
+// Nearest representative of P points per thread.  The representatives lie in
+// shared memory by coordinate, negated (stage_reps), so that four of them come
+// with one 16-byte broadcast read per coordinate and their distances are
+// packed FP32 pairs -- each rounded as dist2_rows rounds it.  The running
+// minimum moves once per four representatives (their minimum first); which of
+// the four it was is found again at the end, so that a representative costs
+// three packed operations (d = 3) and 1.5 others, not six and three.
+// ---------------------------------------------------------------------------
+// Rows reps[0..cnt) of DP4 float4 into s (4 DP4 coordinates, `stride` floats
+// each, a multiple of four >= cnt); up to three rows of NaN, which are nearest
+// to nothing, fill the last four.
+template <int DP4>
+__device__ __forceinline__ void stage_reps(const float4 *__restrict__ reps, int cnt, float *s,
+                                           int stride) {
+  const int full = (cnt + 3) & ~3;
+  const float nan = __int_as_float(0x7fffffff);
+  for (int e = threadIdx.x; e < full * DP4; e += blockDim.x) {
+    const int r = e / DP4, c = e - r * DP4;
+    const float4 v = r < cnt ? reps[(int64_t)r * DP4 + c] : make_float4(nan, nan, nan, nan);
+    s[(4 * c) * stride + r] = -v.x;
+    s[(4 * c + 1) * stride + r] = -v.y;
+    s[(4 * c + 2) * stride + r] = -v.z;
+    s[(4 * c + 3) * stride + r] = -v.w;
+  }
+}
+
+template <int DP4, int P>
+struct NearestRep {
+  float q[P][4 * DP4];
+  float best[P];
+  int quad[P];  // first of the four representatives that hold the minimum
+
+  __device__ __forceinline__ void load(int i, const float4 *__restrict__ row) {
+#pragma unroll
+    for (int c = 0; c < DP4; c++) {
+      const float4 v = row ? row[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+      q[i][4 * c] = v.x;
+      q[i][4 * c + 1] = v.y;
+      q[i][4 * c + 2] = v.z;
+      q[i][4 * c + 3] = v.w;
+    }
+    best[i] = __int_as_float(0x7f7fffff);  // FLT_MAX
+    quad[i] = -1;
+  }
+  // squared distances to representatives j .. j+3
+  __device__ __forceinline__ void four(int i, const float *s, int stride, int j,
+                                       float (&v)[4]) const {
+    float2 v01, v23;
+#pragma unroll
+    for (int c = 0; c < 4 * DP4; c++) {
+      const float4 r = *reinterpret_cast<const float4 *>(s + c * stride + j);
+      const float2 qc = make_float2(q[i][c], q[i][c]);
+      const float2 a = __fadd2_rn(qc, make_float2(r.x, r.y));
+      const float2 b = __fadd2_rn(qc, make_float2(r.z, r.w));
+      v01 = c == 0 ? __fmul2_rn(a, a) : __ffma2_rn(a, a, v01);
+      v23 = c == 0 ? __fmul2_rn(b, b) : __ffma2_rn(b, b, v23);
+    }
+    v[0] = v01.x;
+    v[1] = v01.y;
+    v[2] = v23.x;
+    v[3] = v23.y;
+  }
+  // representatives base .. base + cnt - 1, staged at s
+  __device__ __forceinline__ void scan(const float *s, int stride, int cnt, int base) {
+    for (int j = 0; j < cnt; j += 4) {
+#pragma unroll
+      for (int i = 0; i < P; i++) {
+        float v[4];
+        four(i, s, stride, j, v);
+        const float m = fminf(fminf(v[0], v[1]), fminf(v[2], v[3]));  // ignores NaN
+        if (m < best[i]) {
+          best[i] = m;
+          quad[i] = base + j;
+        }
+      }
+    }
+  }
+};
+
+// The first of representatives quad .. quad+3 (of R) whose squared distance to
+// `row` is `best`: the lowest index on ties.  quad < 0 (no distance was a
+// number): representative 0, a valid cluster.
+template <int DP4>
+__device__ __forceinline__ int nearest_of_quad(const float4 *__restrict__ row,
+                                               const float4 *__restrict__ reps, int R, int quad,
+                                               float best) {
+  if (quad < 0) return 0;
+  float4 p[DP4];
+#pragma unroll
+  for (int c = 0; c < DP4; c++) p[c] = row[c];
+  int b = quad;
+#pragma unroll
+  for (int u = 3; u >= 0; u--)
+    if (quad + u < R && dist2_rows<DP4>(p, reps + (int64_t)(quad + u) * DP4) == best) b = quad + u;
+  return b;
+}
+
 // Warp-cooperative lower bound: first position p in [0, n) of the ascending
 // array a with a[p] >= v (n if none).  32-ary search: each round the lanes
 // sample 32 evenly spaced positions and a ballot brackets the answer, so a
