@@ -507,6 +507,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   a.qrows = Q.Qp;
   a.qorder = Q.qset.perm;
   a.slot_cl = Q.slot_cl;
+  a.qoff = Q.qset.off;
   a.m = nslot;
   a.slot_base = slot0;
   a.d = d;

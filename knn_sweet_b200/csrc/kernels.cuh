@@ -23,6 +23,7 @@ struct ScanArgs {
   const float4 *qrows;      // m x dp4, original query order
   const int32_t *qorder;    // slot -> query row (grouped by query cluster)
   const int32_t *slot_cl;   // slot -> query cluster
+  const int32_t *qoff;      // Rq + 1: first slot of every query cluster
   int64_t m;
   int d, dp4, dp4_tmpl, k;
   bool idx_in_row;          // srows carry the index in their last pad float

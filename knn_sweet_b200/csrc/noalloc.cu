@@ -329,6 +329,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   a.qrows = Qp;
   a.qorder = Qb.perm;
   a.slot_cl = p.slot_cl;
+  a.qoff = Qb.off;
   a.m = m;
   a.d = d;
   a.dp4 = p.dp4s;

@@ -27,6 +27,7 @@
 //   - The k-th boundary is then settled in FP64 (see TopKBase).
 // Bounds are widened by a rounding slack (bound_tol) so that FP32 rounding
 // never prunes a point that the FP32 distances would rank in the top k.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -602,11 +603,6 @@ struct QueryRow<0, IDXROW> {
 #define KNN_INDEX32 1
 #endif
 
-// The thread-per-query scan keeps its statistics counters in shared memory
-// (1) or in registers (0).
-#ifndef KNN_TSCAN_SMEM_STATS
-#define KNN_TSCAN_SMEM_STATS 1
-#endif
 // The query's slot, row and cluster wait out the walk in shared memory (1)
 // or in registers (0).
 #ifndef KNN_SIDE_WORDS
@@ -972,188 +968,477 @@ static int launch_scan_l(const ScanArgs &a, int num_sms, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// Thread-per-query scan for small k (k <= 32) and narrow rows (d <= 8).  With
-// few distances per query (k = 16 on a surface: ~200) the warp-per-query
-// scan spends most of its instructions on per-query and per-cluster overhead
-// (lane-parallel cluster tests, nearest-first ordering, 32-ary band search,
-// list merges) for bands that fill few lanes.  Here every thread walks its own
-// query, in the same order of the same candidate list, with the same pruning
-// tests and the same FP32 keys, keeping its K best keys sorted in registers
-// (K = pow2 >= k; the K-th key is the pruning bound, so for k < K the bound is
-// looser but the first k keys are still the k nearest).  The 32 queries of a
-// warp are consecutive slots, mostly of one query cluster, so they walk
-// similar lists.
-// ---------------------------------------------------------------------------
-template <int K>
-struct ThreadTopK {
-  uint64_t key[K];  // ascending; kKeyMax = empty
-  __device__ __forceinline__ void reset() {
-#pragma unroll
-    for (int j = 0; j < K; j++) key[j] = kKeyMax;
-  }
-  // inserts v, which must be smaller than key[K-1]
-  __device__ __forceinline__ void insert(uint64_t v) {
-#pragma unroll
-    for (int j = K - 1; j > 0; j--) {
-      const uint64_t prev = key[j - 1];
-      key[j] = prev > v ? prev : (key[j] > v ? v : key[j]);
-    }
-    key[0] = key[0] > v ? v : key[0];
-  }
-};
-
-// 4 blocks per SM (64 registers; 71 unbounded gave 3): C4 79.3 -> 76.5 ms.
-// Loading member p + 1 while member p is evaluated measured slower.
+// Group scan for small k (k <= 32) and narrow rows (d <= 8): one warp, up to
+// 32 queries of one query cluster, a query per lane.  The queries share their
+// cluster's candidate list, so the warp walks it once for all of them: every
+// reference cluster that some lane still needs (the scan's own two tests, per
+// lane) contributes the members in the union of those lanes' bands
+// |D - d(s,Rs)| <= theta, 32 at a time through shared memory, and every lane
+// evaluates the same member in the same instruction -- coalesced row loads,
+// broadcast shared-memory reads, no divergence between lanes.
 //
-// FP64 boundary: the pruning bound is band_hi of the K-th key, so every point
-// inside the final k-th's FP32 band is evaluated; one that does not fit the
-// list sets `lost`.  A query whose band reaches behind its k-th (a key inside
+// A candidate (d^2 at most the lane's threshold) goes into the lane's column
+// of a shared-memory buffer; when some lane's column is nearly full, all lanes
+// sort theirs in registers (a fixed network, the same instructions for all)
+// and merge it into their K best keys (K = pow2 >= k), which tightens the
+// lane's threshold.
+//
+// What bounds it: instruction issue (75 % of the slots on 512 surface clouds,
+// k = 16) and the ALU pipe of the merges.  It replaced a thread per query whose
+// every insertion into a sorted list of 64-bit keys was executed by the whole
+// warp: 4,096 surface clouds, k = 16: search 59.4 -> 22.4 ms; 64 pairs of
+// clouds, k = 8 both ways: 3.2 -> 1.4 ms.  64-bit keys in the merges instead
+// of distance words: 32 ms; three blocks per SM (111 registers): 24.2 ms, six
+// (80 registers, spilling): 28 ms.
+//
+// FP64 boundary: the threshold is band_hi of the k-th key, so every point
+// inside the final k-th's FP32 band is evaluated and admitted; one that a merge
+// drops sets `lost`.  A query whose band reaches behind its k-th (a key inside
 // it was lost, or the list holds one after the k-th) goes to the band kernel,
 // which re-decides the band in FP64; on data without near-ties at the k-th
 // that is a small fraction of the queries, and FP64 code stays out of this
 // register-bound kernel.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void order_pair(uint32_t &a, uint32_t &b) {
+  const uint32_t lo = min(a, b), hi = max(a, b);
+  a = lo;
+  b = hi;
+}
+// Keys as doubles: a key's upper word is a float, so no key has a double's
+// exponent of all ones (kLaneEmpty is the largest finite one) and keys order
+// like the doubles of their bits.  One double compare and four selects: 9.3
+// cycles against 16.2 for the integer comparison of two words.
+__device__ __forceinline__ void order_pair(uint64_t &a, uint64_t &b) {
+  const bool sw = __longlong_as_double((long long)a) > __longlong_as_double((long long)b);
+  const uint64_t lo = sw ? b : a, hi = sw ? a : b;
+  a = lo;
+  b = hi;
+}
+constexpr uint64_t kLaneEmpty = 0x7fefffffffffffffull;  // its distance word is a NaN
+
+// Batcher's odd-even merge sort of x[LO .. LO+N) in registers (63 comparators
+// for N = 16).
+template <int LO, int N, int R, class T, int S>
+__device__ __forceinline__ void net_merge(T (&x)[S]) {
+  if constexpr (2 * R < N) {
+    net_merge<LO, N, 2 * R>(x);
+    net_merge<LO + R, N, 2 * R>(x);
+#pragma unroll
+    for (int i = LO + R; i + R < LO + N; i += 2 * R) order_pair(x[i], x[i + R]);
+  } else {
+    order_pair(x[LO], x[LO + R]);
+  }
+}
+template <int LO, int N, class T, int S>
+__device__ __forceinline__ void net_sort(T (&x)[S]) {
+  if constexpr (N > 1) {
+    net_sort<LO, N / 2>(x);
+    net_sort<LO + N / 2, N / 2>(x);
+    net_merge<LO, N, 1>(x);
+  }
+}
+
+// One lane's candidates: a column of (distance, index) words in shared memory
+// (entry j at [32 j]), every candidate up to band_hi of the k-th distance seen
+// among them, and the K smallest distance words in registers, which give that
+// threshold.  Entries [kept, cnt) are not merged into the registers yet.
+constexpr int kLaneNew = 16;  // most entries merged at once
+
+// Keeps the `want` smallest keys of a lane's column of n entries (indices
+// 32 C words behind the distances), in place; returns the smallest distance
+// dropped.  Out of line: only crowds of equal distances come here.
+__device__ __noinline__ float cut_column(uint32_t *col, int C, int n, int want) {
+  float lost = __int_as_float(0x7f800000);
+  auto entry = [&](int j) { return ((uint64_t)col[32 * j] << 32) | col[32 * (C + j)]; };
+  uint64_t keep = 0;
+  for (int e = 0; e < n; e++) {
+    const uint64_t x = entry(e);
+    int rank = 0;
+    for (int f = 0; f < n; f++) rank += entry(f) < x;
+    if (rank < want) keep |= 1ull << e;
+    else lost = fminf(lost, key_d2(x));
+  }
+  int w = 0;
+  for (int e = 0; e < n; e++)
+    if ((keep >> e) & 1) {
+      const uint64_t x = entry(e);
+      col[32 * w] = (uint32_t)(x >> 32);
+      col[32 * (C + w)] = (uint32_t)x;
+      w++;
+    }
+  return lost;
+}
+
+template <int K>
+struct LaneTopK {
+  static constexpr int C = K + kLaneNew;  // column entries
+  uint32_t top[K];  // ascending distance words (all ones: none)
+  uint32_t *col;    // distances; the indices 32 C words further on
+  int kept, cnt;
+  float lost;       // smallest FP32 d^2 dropped for lack of room (+inf: none)
+
+  __device__ __forceinline__ void reset() {
+#pragma unroll
+    for (int j = 0; j < K; j++) top[j] = 0xffffffffu;
+    kept = cnt = 0;
+    lost = __int_as_float(0x7f800000);
+  }
+  __device__ __forceinline__ void push(float v, int32_t idx) {
+    col[32 * cnt] = __float_as_uint(v);
+    col[32 * (C + cnt)] = (uint32_t)idx;
+    cnt++;
+  }
+  // whether some lane may not take four more candidates
+  __device__ __forceinline__ bool crowded() const {
+    return __any_sync(kFull, cnt - kept > kLaneNew - 4 || cnt > C - 4);
+  }
+  // the k-th distance word (selected by masks: a compare-and-select on the
+  // runtime k turns the list into an indexed local-memory array)
+  __device__ __forceinline__ uint32_t at(int i) const {
+    uint32_t r = 0;
+#pragma unroll
+    for (int j = 0; j < K; j++) r |= top[j] & (0u - (uint32_t)(j == i));
+    return r;
+  }
+  __device__ __forceinline__ uint64_t entry(int j) const {
+    return ((uint64_t)col[32 * j] << 32) | col[32 * (C + j)];
+  }
+  // merges the new entries, updates the threshold (squared distances up to
+  // thr enter) and drops the entries above it
+  __device__ __forceinline__ void flush(int k, int d, float &thr) {
+    uint32_t b[kLaneNew];
+#pragma unroll
+    for (int j = 0; j < kLaneNew; j++) {
+      b[j] = 0xffffffffu;
+      if (kept + j < cnt) b[j] = col[32 * (kept + j)];
+    }
+    net_sort<0, kLaneNew>(b);
+    // top ascending, b descending: the minima are the K smallest of both, as
+    // a bitonic sequence
+    constexpr int N = K < kLaneNew ? K : kLaneNew;
+#pragma unroll
+    for (int j = 0; j < N; j++) top[K - 1 - j] = min(top[K - 1 - j], b[j]);
+#pragma unroll
+    for (int s = K / 2; s > 0; s >>= 1) {
+#pragma unroll
+      for (int j = 0; j < K; j++)
+        if ((j & s) == 0) order_pair(top[j], top[j | s]);
+    }
+    const uint32_t kth = k == K ? top[K - 1] : at(k - 1);
+    if (kth != 0xffffffffu) thr = band_hi(__uint_as_float(kth), d);
+    int w = 0;
+    const int most = (int)__reduce_max_sync(kFull, (unsigned)cnt);
+    for (int j0 = 0; j0 < most; j0 += 4) {
+      uint32_t dv[4], iv[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {  // C is a multiple of four
+        dv[u] = col[32 * (j0 + u)];
+        iv[u] = col[32 * (C + j0 + u)];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (j0 + u < cnt && __uint_as_float(dv[u]) <= thr) {
+          col[32 * w] = dv[u];
+          col[32 * (C + w)] = iv[u];
+          w++;
+        }
+    }
+    kept = cnt = w;
+    // many equal distances: the K smallest keys stay
+    if (__any_sync(kFull, kept > C - 8)) cut();
+  }
+  // keeps the K smallest keys of the column; the others go into `lost`
+  __device__ __forceinline__ void cut() {
+    lost = fminf(lost, cut_column(col, C, kept, K));
+    kept = cnt = min(kept, K);
+  }
+};
+
+// warps per block, each on its own group
+__host__ __device__ constexpr int group_warps(int K) { return K > 16 ? 2 : 4; }
+
 template <int DP4, bool IDXROW, int K>
-__global__ void __launch_bounds__(256, 4)
-    thread_scan_kernel(const ScanArgs a) {
-  __shared__ unsigned long long blk_ctr[kScanCounters];
-  if (threadIdx.x < kScanCounters) blk_ctr[threadIdx.x] = 0;
+__global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 : 6))
+    group_scan_kernel(const ScanArgs a) {
+  using TK = LaneTopK<K>;
+  constexpr int kGroupWarps = group_warps(K);
+  __shared__ uint32_t s_col[kGroupWarps][K > 1 ? 2 * TK::C * 32 : 1];
+  // the current 32 members by coordinate (negated); the last pad coordinate
+  // of rows that carry their index there is the index
+  __shared__ __align__(16) float s_mem[kGroupWarps][4 * DP4 + (IDXROW ? 0 : 1)][32];
+  __shared__ float4 s_rep[kGroupWarps][32 * DP4];  // representatives of the list batch
+  __shared__ float4 s_meta[kGroupWarps][32];       // their cmax, cmin, start, size
+  __shared__ unsigned long long blk_ctr[4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x < 4) blk_ctr[threadIdx.x] = 0;
   __syncthreads();
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int d = a.d, k = a.k;
+  const float tol = bound_tol(d);
+  const float inf = __int_as_float(0x7f800000);
+  const bool exact32 = fp32_exact(a);
   const int64_t nslots = a.slot_list ? (int64_t)*a.slot_count : a.m;
-#if KNN_TSCAN_SMEM_STATS
-  // visited, pruned, pushed of this thread's query in shared memory (stride
-  // 3 words: no bank conflicts), out of the walk's registers
-  __shared__ unsigned tstat[3 * 256];
-  unsigned *ts = tstat + 3 * threadIdx.x;
-  ts[0] = ts[1] = ts[2] = 0;
-  unsigned evals = 0;
-#else
+  TK tk;
+  tk.col = &s_col[w][K > 1 ? lane : 0];
   unsigned evals = 0, visited = 0, pruned = 0, pushed = 0;
-#endif
-  if (t < nslots) {
-    const int64_t slot = a.slot_list ? (int64_t)a.slot_list[t] : a.slot_base + t;
-    const int64_t q = a.qorder[slot];
-    const int qc = a.slot_cl[slot];
-    const int d = a.d;
-    const float tol = bound_tol(d);
-    QueryRow<DP4, IDXROW> qr;
-    qr.load(a.qrows, q, DP4, nullptr);
-    ThreadTopK<K> tk;
-    tk.reset();
-    float theta = query_theta0(a, slot, qc, tol);
-    float lost = __int_as_float(0x7f800000);
-    // admits every d^2 <= theta0^2, whatever the index
-    const uint64_t thr0 = ((uint64_t)__float_as_uint(theta * theta) << 32) | 0xffffffffull;
-    const int nr = a.rlen[qc];
-    const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
-    for (int j = 0; j < nr; j++) {
-      const int c = rl[j];
-      const float D = sqrtf(qr.dist2(a.sreps + (int64_t)c * DP4, DP4));
-      float slack = tol * (2.0f * D + 2.0f * theta);
-      const float cmin = a.cmin[c];
-      if (D - a.cmax[c] > theta + slack || D + theta + slack < cmin) {
-#if KNN_TSCAN_SMEM_STATS
-        ts[1]++;
-#else
-        pruned++;
-#endif
+
+  // Windows of 32 slots from the work counter.  Without a slot list a window
+  // stands for the groups that start in it (they begin at every 32nd slot of
+  // their cluster, so no list of groups is needed); with one, for the 32
+  // listed slots, a group per query cluster among them.
+  long long s = 0, s_end = 0, c0 = 0, c1 = 0;
+  int qc = 0, listed_qc = -1;
+  unsigned todo = 0;
+  for (;;) {
+    int64_t slot;
+    bool act;
+    if (a.slot_list ? todo == 0 : s >= s_end) {
+      long long win = 0;
+      if (lane == 0) win = (long long)atomicAdd(a.work_counter, 1ull);
+      win = __shfl_sync(kFull, win, 0) * 32;
+      if (win >= nslots) break;
+      s = a.slot_base + win;
+      s_end = min(s + 32, (long long)a.slot_base + (long long)nslots);
+      if (a.slot_list) {
+        const bool have = win + lane < nslots;
+        s = have ? a.slot_list[win + lane] : 0;
+        listed_qc = have ? a.slot_cl[s] : -1;
+        todo = __ballot_sync(kFull, have);
+      } else {
+        qc = a.slot_cl[s];
+        c0 = a.qoff[qc];
+        c1 = a.qoff[qc + 1];
+        s = min(c0 + ((s - c0 + 31) & ~31ll), c1);
         continue;
       }
-#if KNN_TSCAN_SMEM_STATS
-      ts[0]++;
-#else
-      visited++;
-#endif
-      const int start = a.soff[c], n_c = a.soff[c + 1] - start;
-      const float *sd = a.sdist + start;
-      // first member of the band [D - theta, D + theta] (with slack)
-      const float lo_edge = D - theta - slack;
-      int p = 0;
-      if (lo_edge > cmin) {
-        int hi = n_c;
-        while (p < hi) {
-          const int md = (p + hi) >> 1;
-          if (sd[md] < lo_edge) p = md + 1;
-          else hi = md;
-        }
+    }
+    if (a.slot_list) {
+      qc = __shfl_sync(kFull, listed_qc, __ffs((int)todo) - 1);
+      slot = s;
+      act = listed_qc == qc;
+      todo &= ~__ballot_sync(kFull, act);
+    } else {
+      if (s == c1) {  // the next cluster with queries
+        qc = a.slot_cl[s];
+        c1 = a.qoff[qc + 1];
       }
-      for (; p < n_c; p++) {
-        if (sd[p] > D + theta + slack) break;
-        float4 row[DP4];
+      slot = s + lane;
+      act = slot < c1;
+      s = min(s + 32, c1);
+    }
+    // one group: lane's query slot (act: it has one), all of query cluster qc
+    const int64_t q = act ? a.qorder[slot] : 0;
+    QueryRow<DP4, IDXROW> qr;
+    qr.load(a.qrows, q, DP4, nullptr);
+    constexpr int kCoords = 4 * DP4 - (IDXROW ? 1 : 0);
+    float2 qq[4 * DP4];
 #pragma unroll
-        for (int cc = 0; cc < DP4; cc++) row[cc] = a.srows[(int64_t)(start + p) * DP4 + cc];
-        int32_t idx = 0;
-        const float v = qr.dist2_member(row, &idx);
-        evals++;
-        if (!IDXROW) idx = a.sidx[start + p];
-        const uint64_t key = make_key(v, idx);
-        if (key < thr0) {
-          if (key < tk.key[K - 1]) {
-            lost = fminf(lost, key_d2(tk.key[K - 1]));  // NaN (empty) is ignored
-            tk.insert(key);
-#if KNN_TSCAN_SMEM_STATS
-            ts[2]++;
-#else
-            pushed++;
-#endif
-            if (tk.key[K - 1] != kKeyMax) {
-              theta = sqrtf(band_hi(key_d2(tk.key[K - 1]), d));
-              slack = tol * (2.0f * D + 2.0f * theta);
-            }
+    for (int e = 0; e < DP4; e++) {
+      qq[4 * e] = make_float2(qr.v[e].x, qr.v[e].x);
+      qq[4 * e + 1] = make_float2(qr.v[e].y, qr.v[e].y);
+      qq[4 * e + 2] = make_float2(qr.v[e].z, qr.v[e].z);
+      qq[4 * e + 3] = make_float2(qr.v[e].w, qr.v[e].w);
+    }
+    tk.reset();
+    uint64_t best = kLaneEmpty;  // the list for k = 1
+    float theta = act ? query_theta0(a, slot, qc, tol) : 0.0f;
+    float thr = theta * theta;  // admits every d^2 <= theta0^2, whatever the index
+    const int nr = a.rlen[qc];
+    const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
+    for (int base = 0; base < nr; base += 32) {
+      const int nb = min(32, nr - base);
+      __syncwarp();
+      if (lane < nb) {
+        const int c = rl[base + lane];
+#pragma unroll
+        for (int e = 0; e < DP4; e++) s_rep[w][lane * DP4 + e] = a.sreps[(int64_t)c * DP4 + e];
+        const int st = a.soff[c];
+        s_meta[w][lane] = make_float4(a.cmax[c], a.cmin[c], __int_as_float(st),
+                                      __int_as_float(a.soff[c + 1] - st));
+      }
+      __syncwarp();
+      for (int i = 0; i < nb; i++) {
+        const float D = sqrtf(qr.dist2(&s_rep[w][i * DP4], DP4));
+        const float4 mt = s_meta[w][i];
+        float slack = tol * (2.0f * D + 2.0f * theta);
+        const bool need = act && !(D - mt.x > theta + slack || D + theta + slack < mt.y);
+        visited += need;
+        pruned += act && !need;
+        if (!__any_sync(kFull, need)) continue;
+        // the union of the lanes' bands; a NaN edge (a lane whose distances
+        // are not numbers) opens the band instead of closing it
+        const float lo_l = D - theta - slack, hi_l = D + theta + slack;
+        const float lo = __uint_as_float(__reduce_min_sync(
+            kFull, __float_as_uint(need ? fmaxf(lo_l, 0.0f) : inf)));
+        const float hi = __uint_as_float(__reduce_max_sync(
+            kFull, __float_as_uint(need ? (hi_l < inf ? fmaxf(hi_l, 0.0f) : inf) : 0.0f)));
+        float cut = need ? thr : -1.0f;  // no d^2 passes a lane that is done with c
+        const int start = __float_as_int(mt.z), n_c = __float_as_int(mt.w);
+        for (int c0 = 0; c0 < n_c; c0 += 32) {
+          const int p = c0 + lane;
+          const bool valid = p < n_c;
+          const unsigned gp = (unsigned)(start + p);
+          float4 row[DP4];
+          float ds = inf;
+          if (valid) {
+            ds = a.sdist[gp];
+#pragma unroll
+            for (int e = 0; e < DP4; e++) row[e] = a.srows[(size_t)gp * DP4 + e];
           } else {
-            lost = fminf(lost, v);
+            // a row that passes no lane: its distances are NaN
+#pragma unroll
+            for (int e = 0; e < DP4; e++)
+              row[e] = make_float4(__int_as_float(0x7fffffff), 0.0f, 0.0f, 0.0f);
           }
+          const bool inb = valid && ds >= lo && !(ds > hi);
+          const unsigned bm = __ballot_sync(kFull, inb);
+          const bool last = __ballot_sync(kFull, valid && !(ds > hi)) != kFull;
+          if (bm) {
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < DP4; e++) {
+              s_mem[w][4 * e][lane] = -row[e].x;
+              s_mem[w][4 * e + 1][lane] = -row[e].y;
+              s_mem[w][4 * e + 2][lane] = -row[e].z;
+              s_mem[w][4 * e + 3][lane] = IDXROW && e == DP4 - 1 ? row[e].w : -row[e].w;
+            }
+            if constexpr (!IDXROW)
+              s_mem[w][4 * DP4][lane] = valid ? __int_as_float(a.sidx[gp]) : 0.0f;
+            __syncwarp();
+            const int p1 = 31 - __clz((int)bm);
+            const int p0 = (__ffs((int)bm) - 1) & ~3;
+            // four members at a time (the few outside the band that this
+            // rounds in are members too: their distances are as good)
+            for (int t = p0; t <= p1; t += 4) {
+              // packed FP32 pairs, the scan's arithmetic for each member
+              float2 v01, v23;
+#pragma unroll
+              for (int c = 0; c < kCoords; c++) {
+                const float4 s4 = *reinterpret_cast<const float4 *>(&s_mem[w][c][t]);
+                const float2 d01 = __fadd2_rn(qq[c], make_float2(s4.x, s4.y));
+                const float2 d23 = __fadd2_rn(qq[c], make_float2(s4.z, s4.w));
+                v01 = c == 0 ? __fmul2_rn(d01, d01) : __ffma2_rn(d01, d01, v01);
+                v23 = c == 0 ? __fmul2_rn(d23, d23) : __ffma2_rn(d23, d23, v23);
+              }
+              const float v[4] = {v01.x, v01.y, v23.x, v23.y};
+              const float4 id4 = *reinterpret_cast<const float4 *>(&s_mem[w][kCoords][t]);
+              const int32_t id[4] = {__float_as_int(id4.x), __float_as_int(id4.y),
+                                     __float_as_int(id4.z), __float_as_int(id4.w)};
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                if (v[u] <= cut) {
+                  if constexpr (K > 1) {
+                    tk.push(v[u], id[u]);
+                  } else {
+                    const uint64_t key = make_key(v[u], id[u]);
+                    tk.lost = fminf(tk.lost, key_d2(umax64(best, key)));
+                    best = umin64(best, key);
+                    pushed++;
+                  }
+                }
+              }
+              if constexpr (K > 1) {
+                if (tk.crowded()) {
+                  pushed += tk.cnt - tk.kept;
+                  tk.flush(k, d, thr);
+                  if (need) cut = thr;
+                }
+              } else if (best != kLaneEmpty) {
+                thr = band_hi(key_d2(best), d);
+                if (need) cut = thr;
+              }
+            }
+            if (need) evals += (unsigned)(p1 - p0 + 1);
+          }
+          if (last) break;
+        }
+        theta = fminf(theta, sqrtf(thr));
+      }
+    }
+    // the K best keys, ascending
+    uint64_t key[K];
+    if constexpr (K > 1) {
+      if (__any_sync(kFull, tk.cnt > tk.kept)) {
+        pushed += tk.cnt - tk.kept;
+        tk.flush(k, d, thr);
+      }
+      if (__any_sync(kFull, tk.kept > K)) tk.cut();
+#pragma unroll
+      for (int j = 0; j < K; j++) {
+        key[j] = kLaneEmpty;
+        if (j < tk.kept) key[j] = tk.entry(j);
+      }
+      net_sort<0, K>(key);
+    } else {
+      key[0] = best;
+    }
+    if (act) {
+      // the k-th key, the key behind it, and the FP32 band around the k-th
+      uint64_t kth = 0, next = 0;
+#pragma unroll
+      for (int j = 0; j < K; j++) {
+        kth |= key[j] & (0ull - (uint64_t)(j == k - 1));
+        next |= key[j] & (0ull - (uint64_t)(j == k));
+      }
+      if (k >= K) next = kLaneEmpty;
+      bool defer = false;
+      int nlo = 0;
+      const float Dk = key_d2(kth);
+      if (kth != kLaneEmpty && !exact32) {
+        const float bhi = band_hi(Dk, d);
+        // a band key was dropped, or one sits behind the k-th (NaN: none)
+        defer = tk.lost <= bhi || key_d2(next) <= bhi;
+        if (defer) {
+          const float blo = band_lo(Dk, d);
+#pragma unroll
+          for (int j = 0; j < K; j++) nlo += key_d2(key[j]) < blo;
         }
       }
-    }
-    // the k-th key, the key behind it, and the FP32 band around the k-th
-    // (selected by masks: a compare-and-select on the runtime k turns the
-    // list into an indexed local-memory array)
-    uint64_t kth = 0, next = 0;
+      int32_t *oi = a.out_idx + q * k;
+      float *od = a.out_dist + q * k;
+      const int32_t rbase = a.qc_ref_base ? (int32_t)a.qc_ref_base[qc] : 0;
+      auto idx_of = [&](uint64_t x) {
+        return x == kLaneEmpty ? -1 : key_idx(x) - rbase;
+      };
+      auto dist_of = [&](uint64_t x) {
+        const float d2 = key_d2(x);
+        return x == kLaneEmpty ? inf : (a.squared ? d2 : sqrtf(d2));
+      };
+      bool quads = false;
+      if constexpr (K >= 4)
+        quads = (k & 3) == 0 &&
+                ((reinterpret_cast<uintptr_t>(a.out_idx) | reinterpret_cast<uintptr_t>(a.out_dist)) &
+                 15) == 0;
+      if (quads) {
+        if constexpr (K >= 4) {
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-      kth |= tk.key[j] & (0ull - (uint64_t)(j == a.k - 1));
-      next |= tk.key[j] & (0ull - (uint64_t)(j == a.k));
-    }
-    if (a.k >= K) next = kKeyMax;
-    bool defer = false;
-    int nlo = 0;
-    const float Dk = key_d2(kth);
-    if (kth != kKeyMax && !fp32_exact(a)) {
-      const float hi = band_hi(Dk, d);
-      // a band key was dropped, or one sits behind the k-th (NaN: none)
-      defer = lost <= hi || key_d2(next) <= hi;
+          for (int j = 0; j < K; j += 4)
+            if (j < k) {
+              *reinterpret_cast<int4 *>(oi + j) = make_int4(
+                  idx_of(key[j]), idx_of(key[j + 1]), idx_of(key[j + 2]),
+                  idx_of(key[j + 3]));
+              *reinterpret_cast<float4 *>(od + j) = make_float4(
+                  dist_of(key[j]), dist_of(key[j + 1]), dist_of(key[j + 2]),
+                  dist_of(key[j + 3]));
+            }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < K; j++)
+          if (j < k) {
+            oi[j] = idx_of(key[j]);
+            od[j] = dist_of(key[j]);
+          }
+      }
       if (defer) {
-        const float lo = band_lo(Dk, d);
-#pragma unroll
-        for (int j = 0; j < K; j++) nlo += key_d2(tk.key[j]) < lo;
+        // the band kernel settles the boundary: it reads the number of keys
+        // below the band and the k-th value from the last slot
+        oi[k - 1] = nlo;
+        od[k - 1] = Dk;
+        a.unres_slot[atomicAdd(a.unres_count, 1u)] = (int32_t)slot;
       }
-    }
-    int32_t *oi = a.out_idx + q * a.k;
-    float *od = a.out_dist + q * a.k;
-    const int32_t base = a.qc_ref_base ? (int32_t)a.qc_ref_base[qc] : 0;
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-      if (j < a.k) {
-        const uint64_t key = tk.key[j];
-        const bool none = key == kKeyMax;
-        oi[j] = none ? -1 : key_idx(key) - base;
-        const float d2 = key_d2(key);
-        od[j] = none ? __int_as_float(0x7f800000) : (a.squared ? d2 : sqrtf(d2));
-      }
-    }
-    if (defer) {
-      // the band kernel settles the boundary: it reads the number of keys
-      // below the band and the k-th value from the last slot
-      oi[a.k - 1] = nlo;
-      od[a.k - 1] = Dk;
-      a.unres_slot[atomicAdd(a.unres_count, 1u)] = (int32_t)slot;
     }
   }
   if (a.counters) {
-#if KNN_TSCAN_SMEM_STATS
-    unsigned visited = ts[0], pruned = ts[1], pushed = ts[2];
-#endif
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       evals += __shfl_xor_sync(kFull, evals, o);
@@ -1161,37 +1446,40 @@ __global__ void __launch_bounds__(256, 4)
       pruned += __shfl_xor_sync(kFull, pruned, o);
       pushed += __shfl_xor_sync(kFull, pushed, o);
     }
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
       atomicAdd(&blk_ctr[0], (unsigned long long)evals);
       atomicAdd(&blk_ctr[1], (unsigned long long)visited);
       atomicAdd(&blk_ctr[2], (unsigned long long)pruned);
       atomicAdd(&blk_ctr[3], (unsigned long long)pushed);
     }
     __syncthreads();
-    if (threadIdx.x < kScanCounters) atomicAdd(a.counters + threadIdx.x, blk_ctr[threadIdx.x]);
+    if (threadIdx.x < 4) atomicAdd(a.counters + threadIdx.x, blk_ctr[threadIdx.x]);
   }
 }
 
 template <int DP4, bool IDXROW>
-static int launch_thread_scan(const ScanArgs &a, cudaStream_t s) {
-  const int blocks = (int)((a.m + 255) / 256);
-  auto go = [&](auto kern) -> int {
-    kern<<<blocks, 256, 0, s>>>(a);
+static int launch_group_scan(const ScanArgs &a, int num_sms, cudaStream_t s) {
+  auto go = [&](auto kern, int warps) -> int {
+    int per_sm = 0;
+    KNN_CUDA_TRY(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, 0));
+    const int64_t want = (a.m + 32 * warps - 1) / (32 * warps);
+    const int64_t grid = std::min<int64_t>((int64_t)num_sms * std::max(per_sm, 1), want);
+    kern<<<(unsigned)std::max<int64_t>(grid, 1), warps * 32, 0, s>>>(a);
     KNN_LAUNCH_CHECK();
     return KNN_OK;
   };
-  if (a.k <= 1) return go(thread_scan_kernel<DP4, IDXROW, 1>);
-  if (a.k <= 2) return go(thread_scan_kernel<DP4, IDXROW, 2>);
-  if (a.k <= 4) return go(thread_scan_kernel<DP4, IDXROW, 4>);
-  if (a.k <= 8) return go(thread_scan_kernel<DP4, IDXROW, 8>);
-  if (a.k <= 16) return go(thread_scan_kernel<DP4, IDXROW, 16>);
-  return go(thread_scan_kernel<DP4, IDXROW, 32>);
+  if (a.k <= 1) return go(group_scan_kernel<DP4, IDXROW, 1>, group_warps(1));
+  if (a.k <= 4) return go(group_scan_kernel<DP4, IDXROW, 4>, group_warps(4));
+  if (a.k <= 8) return go(group_scan_kernel<DP4, IDXROW, 8>, group_warps(8));
+  if (a.k <= 16) return go(group_scan_kernel<DP4, IDXROW, 16>, group_warps(16));
+  return go(group_scan_kernel<DP4, IDXROW, 32>, group_warps(32));
 }
 
 // ---------------------------------------------------------------------------
 // Band kernel: the k-th boundary of the queries the scan kernels could not
 // settle (a key of the final band was dropped for lack of room, or the
-// thread scan's list holds one behind the k-th).  One block per query, over
+// group scan's list holds one behind the k-th).  One block per query, over
 // the same candidate list: every point whose FP32 d^2 -- computed with the
 // scan's own arithmetic, so the values are the same -- lies inside the band
 // band_lo(Dk) .. band_hi(Dk) of the k-th is found again, and the band's
@@ -1370,10 +1658,6 @@ static int launch_band_resolve(const ScanArgs &a, int num_sms, cudaStream_t s) {
   return KNN_OK;
 }
 
-#ifndef KNN_THREAD_SCAN_MAX_K
-#define KNN_THREAD_SCAN_MAX_K 32
-#endif
-
 static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s);
 
 // The scan of one batch of query slots, then the band kernel for the queries
@@ -1391,16 +1675,16 @@ int launch_scan(const ScanArgs &a, int num_sms, cudaStream_t s) {
 }
 
 static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
-  // thread per query: small k, rows of at most 8 floats, and short bands (at
-  // most 128 points per cluster on average).  Measured: 4,096 surface clouds
-  // (~70-100 points per cluster, k = 16) 143 -> 67 ms; a dense 3-D set with
-  // ~300 points per cluster at k = 32 2.7 -> 4.3 ms (slower); d = 16 and 32
-  // slower too.
+  // group scan: small k, rows of at most 8 floats, and short bands (at most
+  // 128 points per cluster on average); with longer ones the warp per query
+  // skips more of a cluster than a group of queries can
   const bool short_bands = a.n_ref > 0 && a.Rs > 0 && a.n_ref <= 128 * (int64_t)a.Rs;
-  if (a.k <= KNN_THREAD_SCAN_MAX_K && short_bands && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
+  if (a.k <= 32 && short_bands && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
-      return a.idx_in_row ? launch_thread_scan<1, true>(a, s) : launch_thread_scan<1, false>(a, s);
-    return a.idx_in_row ? launch_thread_scan<2, true>(a, s) : launch_thread_scan<2, false>(a, s);
+      return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)
+                          : launch_group_scan<1, false>(a, num_sms, s);
+    return a.idx_in_row ? launch_group_scan<2, true>(a, num_sms, s)
+                        : launch_group_scan<2, false>(a, num_sms, s);
   }
   switch (a.dp4_tmpl) {
     case 1: return a.idx_in_row ? launch_scan_l<1, true>(a, num_sms, s)
