@@ -321,8 +321,18 @@ int build_ref_side(Arena &keep, Arena &tmp, const float *r, int64_t n, int d, in
   KNN_TRY(keep.alloc(&R->cmax, (size_t)Rs));
   // rows with a spare pad float carry their index there (register-width rows)
   R->idx_in_row = R->tmpl > 0 && 4 * dp4s > d;
-  KNN_TRY(launch_cluster_layout(R->sset.skeys, R->sset.perm, n, R->Rp, dp4s, R->idx_in_row,
-                                R->srows, R->sdist, R->sidx, s));
+  const int32_t *order = R->sset.perm;
+  if (narrow_rows(R->tmpl)) {
+    KNN_TRY(keep.alloc(&R->order, (size_t)n));
+    KNN_TRY(keep.alloc(&R->boxes, (size_t)block_count(n, Rs) * 2 * dp4s));
+    KNN_TRY(launch_block_order(R->Rp, dp4s, d, R->sset.reps, R->sset.skeys, R->sset.off,
+                               R->sset.perm, n, R->order, s));
+    order = R->order;
+  }
+  KNN_TRY(launch_cluster_layout(R->sset.skeys, order, n, R->Rp, dp4s, R->idx_in_row, R->srows,
+                                R->sdist, R->sidx, s));
+  if (R->boxes)
+    KNN_TRY(launch_block_boxes(R->srows, dp4s, d, R->sset.skeys, R->sset.off, n, R->boxes, s));
   KNN_TRY(launch_cluster_minmax(R->sset.off, R->sdist, Rs, R->cmin, R->cmax, s));
   return KNN_OK;
 }
@@ -396,6 +406,7 @@ int build_query_side(const RefSide &R, bool share, const float *q, int64_t m, in
   if (share) {
     Q->Qp = R.Rp;
     Q->qset = R.sset;
+    Q->order = R.order ? R.order : R.sset.perm;
   } else {
     if (dp4s * 4 == d && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
       Q->Qp = reinterpret_cast<const float4 *>(q);
@@ -410,6 +421,14 @@ int build_query_side(const RefSide &R, bool share, const float *q, int64_t m, in
     Q->inexact = qf;
     KNN_TRY(build_clusters(ar, ar, Q->Qp, m, d, dp4s, Rq, o.seed, o.rep_trials, o.lloyd_iters,
                            use_tc, dev_err, s, &Q->qset));
+    Q->order = Q->qset.perm;
+    if (narrow_rows(R.tmpl)) {
+      int32_t *order;
+      KNN_TRY(ar.alloc(&order, (size_t)m));
+      KNN_TRY(launch_block_order(Q->Qp, dp4s, d, Q->qset.reps, Q->qset.skeys, Q->qset.off,
+                                 Q->qset.perm, m, order, s));
+      Q->order = order;
+    }
   }
   KNN_TRY(ar.alloc(&Q->qrad, (size_t)Rq));
   KNN_TRY(ar.alloc(&Q->slot_cl, (size_t)m));
@@ -505,7 +524,9 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
 
   ScanArgs a{};
   a.qrows = Q.Qp;
-  a.qorder = Q.qset.perm;
+  a.qorder = Q.order;
+  a.qreps = Q.qset.reps;
+  a.boxes = R.boxes;
   a.slot_cl = Q.slot_cl;
   a.qoff = Q.qset.off;
   a.m = nslot;
@@ -587,7 +608,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
     KNN_TRY(ar.alloc(&cwork, (size_t)nchunks));
     KNN_CUDA_TRY(cudaMemsetAsync(cwork, 0, nchunks * sizeof(unsigned long long), s));
     KNN_TRY(upload_i32(counts, ccount, s));
-    KNN_TRY(launch_chunk_slots(Q.qset.perm, m, (int)first, chunk_rows, nchunks, ckeys, ckeys_out,
+    KNN_TRY(launch_chunk_slots(Q.order, m, (int)first, chunk_rows, nchunks, ckeys, ckeys_out,
                                cvals, cslots, ctemp, tb, s));
     std::vector<cudaEvent_t> *evs;
     KNN_TRY(chunk_events(nchunks, &evs));

@@ -340,6 +340,7 @@ struct BatchSide {
   uint64_t *skeys = nullptr;
   int32_t *perm = nullptr;
   int32_t *off = nullptr;   // Rtot + 1
+  int32_t *order = nullptr; // slot -> row as the scan takes it (narrow rows: block order)
 };
 
 int cluster_side(BatchArena &ar, const float *pts, const int64_t *off_h, int ncloud, int d,
@@ -421,6 +422,11 @@ int cluster_side(BatchArena &ar, const float *pts, const int64_t *off_h, int ncl
                               b->perm, temp, temp_bytes, s));
   KNN_TRY(ar.alloc(&b->off, (size_t)b->Rtot + 1));
   KNN_TRY(launch_cluster_offsets(b->skeys, b->total, b->Rtot, b->off, s));
+  b->order = b->perm;
+  // (in place: nothing reads the order by distance after this)
+  if (narrow_rows(dp4))
+    KNN_TRY(launch_block_order(b->rows, dp4, d, b->reps, b->skeys, b->off, b->perm, b->total,
+                               b->order, s));
   return KNN_OK;
 }
 
@@ -488,9 +494,14 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       KNN_TRY(ar.alloc(&cmin, (size_t)S.Rtot + 1));
       KNN_TRY(ar.alloc(&cmax, (size_t)S.Rtot + 1));
       const bool idx_in_row = 4 * dp4 > d;
-      KNN_TRY(launch_cluster_layout(S.skeys, S.perm, n, S.rows, dp4, idx_in_row, srows, sdist,
+      KNN_TRY(launch_cluster_layout(S.skeys, S.order, n, S.rows, dp4, idx_in_row, srows, sdist,
                                     sidx, s));
       KNN_TRY(launch_cluster_minmax(S.off, sdist, S.Rtot, cmin, cmax, s));
+      float4 *boxes = nullptr;
+      if (narrow_rows(dp4)) {
+        KNN_TRY(ar.alloc(&boxes, (size_t)block_count(n, S.Rtot) * 2 * dp4));
+        KNN_TRY(launch_block_boxes(srows, dp4, d, S.skeys, S.off, n, boxes, s));
+      }
       if (self) {
         Q = S;
       } else {
@@ -546,7 +557,9 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       if (st) KNN_CUDA_TRY(cudaEventRecord(ev[1], s));
       ScanArgs a{};
       a.qrows = Q.rows;
-      a.qorder = Q.perm;
+      a.qorder = Q.order;
+      a.qreps = Q.reps;
+      a.boxes = boxes;
       a.slot_cl = slot_cl;
       a.qoff = Q.off;
       a.m = m;

@@ -8,6 +8,8 @@
 //   cluster_keys_kernel    (cluster, distance) sort keys
 //   cluster_layout_kernel  cluster-contiguous, distance-sorted copy of the rows
 //   cluster_bounds_kernel  cluster offsets, min/max member distance
+//   block_order_kernel     narrow rows: members near one another next to one
+//   block_boxes_kernel     another, bounding boxes of blocks of 32
 //   rep_dist_kernel        representative-to-representative distances
 //   bounds_filter_kernel   per query cluster: k-th upper bound + surviving
 //                          reference clusters sorted by rep-rep distance
@@ -454,6 +456,169 @@ __global__ void slot_cluster_kernel(const uint64_t *__restrict__ skeys,
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m;
        p += (int64_t)gridDim.x * blockDim.x)
     slot_cl[p] = (int32_t)(skeys[p] >> 32);
+}
+
+// ---------------------------------------------------------------------------
+// Block order of narrow rows.  The sort leaves a cluster's members by their
+// distance to the representative, so that 32 consecutive ones form a shell
+// around it; for rows of few coordinates 32 neighbours in space are a far
+// tighter set, and the scans of narrow rows skip blocks of 32 by their
+// bounding box.  Here every run of 1,024 positions is reordered, cluster by
+// cluster, along a Morton curve over the cluster's own extent (the ball of its
+// radius around its representative); a cluster that crosses a run's end is
+// ordered in parts.  One block per run, keys in shared memory: cluster (less
+// the run's first), Morton code, position.
+// ---------------------------------------------------------------------------
+constexpr int kOrderRun = 1024;
+
+template <int DP4>
+__global__ void __launch_bounds__(kOrderRun / 2)
+    block_order_kernel(const float4 *__restrict__ rows, int d, const float4 *__restrict__ reps,
+                       const uint64_t *__restrict__ skeys, const int32_t *__restrict__ off,
+                       const int32_t *perm, int64_t n, int32_t *out) {
+  __shared__ uint64_t key[kOrderRun];
+  __shared__ int32_t src[kOrderRun];
+  const int64_t base = (int64_t)blockIdx.x * kOrderRun;
+  const int cnt = (int)min((int64_t)kOrderRun, n - base);
+  const int c_first = (int)(skeys[base] >> 32);
+  const int bits = min(10, 30 / d);  // per coordinate
+  const float top = (float)((1 << bits) - 1);
+  for (int t = threadIdx.x; t < kOrderRun; t += blockDim.x) {
+    uint64_t k = kKeyMax;
+    if (t < cnt) {
+      const int c = (int)(skeys[base + t] >> 32);
+      const int32_t row = perm[base + t];
+      const float rad = __uint_as_float((uint32_t)skeys[off[c + 1] - 1]);
+      const float scale = rad > 0.0f ? 0.5f * top / rad : 0.0f;
+      float x[4 * DP4];
+#pragma unroll
+      for (int e = 0; e < DP4; e++) {
+        const float4 v = rows[(int64_t)row * DP4 + e], r = reps[(int64_t)c * DP4 + e];
+        x[4 * e] = v.x - r.x;
+        x[4 * e + 1] = v.y - r.y;
+        x[4 * e + 2] = v.z - r.z;
+        x[4 * e + 3] = v.w - r.w;
+      }
+      uint32_t code = 0;
+#pragma unroll
+      for (int e = 0; e < 4 * DP4; e++)
+        if (e < d) {
+          // (a NaN becomes 0: such a row may go anywhere)
+          const int q = (int)fminf(fmaxf(x[e] * scale + 0.5f * top, 0.0f), top);
+          for (int b = 0; b < bits; b++) code |= (uint32_t)((q >> b) & 1) << (b * d + e);
+        }
+      k = ((uint64_t)(uint32_t)(c - c_first) << 40) | ((uint64_t)code << 10) | (uint32_t)t;
+      src[t] = row;
+    }
+    key[t] = k;
+  }
+  int p2 = 32;
+  while (p2 < cnt) p2 <<= 1;
+  __syncthreads();
+  for (int size = 2; size <= p2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const int t = threadIdx.x;
+      if (t < p2 / 2) {
+        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+        const bool up = (i & size) == 0;
+        const uint64_t a = key[i], b = key[j];
+        if ((a > b) == up) {
+          key[i] = b;
+          key[j] = a;
+        }
+      }
+      // strides below a warp's 64 keys stay inside the warp
+      if (stride > 32) __syncthreads();
+      else __syncwarp();
+    }
+    __syncthreads();
+  }
+  for (int t = threadIdx.x; t < cnt; t += blockDim.x) out[base + t] = src[(int)(key[t] & 1023u)];
+}
+
+// Bounding boxes of the blocks of 32 rows: a warp per 32 positions, for the
+// blocks that start among them (a cluster's blocks start at every 32nd of its
+// positions).  Coordinates from d on (padding, the row index) get 0 .. 0.
+template <int DP4>
+__global__ void __launch_bounds__(256)
+    block_boxes_kernel(const float4 *__restrict__ srows, int d,
+                       const uint64_t *__restrict__ skeys, const int32_t *__restrict__ off,
+                       int64_t n, float4 *__restrict__ boxes) {
+  const int lane = threadIdx.x & 31;
+  const int64_t win = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+  if (win >= n) return;
+  const int64_t end = min(win + 32, n);
+  int c = (int)(skeys[win] >> 32);
+  int64_t c0 = off[c], c1 = off[c + 1];
+  int64_t s = min(c0 + ((win - c0 + 31) & ~(int64_t)31), c1);
+  while (s < end) {
+    if (s == c1) {  // the next cluster with members
+      c = (int)(skeys[s] >> 32);
+      c0 = s;
+      c1 = off[c + 1];
+    }
+    const float inf = __int_as_float(0x7f800000);
+    float lo[4 * DP4], hi[4 * DP4];
+#pragma unroll
+    for (int e = 0; e < DP4; e++) {
+      const bool in = s + lane < c1;
+      const float4 v = in ? srows[(s + lane) * DP4 + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        lo[4 * e + u] = in ? x[u] : inf;
+        hi[4 * e + u] = in ? x[u] : -inf;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4 * DP4; e++) {
+      if (e < d) {  // fminf / fmaxf ignore NaN: no distance to such a row is a number
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          lo[e] = fminf(lo[e], __shfl_xor_sync(kFull, lo[e], o));
+          hi[e] = fmaxf(hi[e], __shfl_xor_sync(kFull, hi[e], o));
+        }
+      } else {
+        lo[e] = hi[e] = 0.0f;
+      }
+    }
+    if (lane == 0) {
+      float4 *b = boxes + (block_slot(c0, c) + (s - c0) / 32) * 2 * DP4;
+#pragma unroll
+      for (int e = 0; e < DP4; e++) {
+        b[e] = make_float4(lo[4 * e], lo[4 * e + 1], lo[4 * e + 2], lo[4 * e + 3]);
+        b[DP4 + e] = make_float4(hi[4 * e], hi[4 * e + 1], hi[4 * e + 2], hi[4 * e + 3]);
+      }
+    }
+    s = min(s + 32, c1);
+  }
+}
+
+bool narrow_rows(int dp4) { return dp4 == 1 || dp4 == 2; }
+
+int launch_block_order(const float4 *rows, int dp4, int d, const float4 *reps,
+                       const uint64_t *skeys, const int32_t *off, const int32_t *perm, int64_t n,
+                       int32_t *out, cudaStream_t s) {
+  if (n == 0) return KNN_OK;
+  const unsigned blocks = (unsigned)((n + kOrderRun - 1) / kOrderRun);
+  if (dp4 == 1)
+    block_order_kernel<1><<<blocks, kOrderRun / 2, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
+  else
+    block_order_kernel<2><<<blocks, kOrderRun / 2, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
+  KNN_LAUNCH_CHECK();
+  return KNN_OK;
+}
+
+int launch_block_boxes(const float4 *srows, int dp4, int d, const uint64_t *skeys,
+                       const int32_t *off, int64_t n, float4 *boxes, cudaStream_t s) {
+  if (n == 0) return KNN_OK;
+  const unsigned blocks = (unsigned)((n + 255) / 256);
+  if (dp4 == 1)
+    block_boxes_kernel<1><<<blocks, 256, 0, s>>>(srows, d, skeys, off, n, boxes);
+  else
+    block_boxes_kernel<2><<<blocks, 256, 0, s>>>(srows, d, skeys, off, n, boxes);
+  KNN_LAUNCH_CHECK();
+  return KNN_OK;
 }
 
 // d(Rq_a, Rs_b) for all pairs (the reference recomputes these inside

@@ -28,8 +28,13 @@ struct ScanArgs {
   int d, dp4, dp4_tmpl, k;
   bool idx_in_row;          // srows carry the index in their last pad float
   bool squared;             // write squared distances instead of distances
+  const float4 *qreps;      // Rq x dp4 query representatives (narrow rows)
   const float4 *sreps;      // Rs x dp4 reference representatives
-  const float4 *srows;      // n x dp4, cluster-contiguous, ascending d(s,Rs)
+  const float4 *srows;      // n x dp4, cluster-contiguous: ascending d(s,Rs),
+                            // or (narrow rows) in block order
+  const float4 *boxes;      // narrow rows: per block of 32 rows of a cluster the
+                            // corners of its bounding box (block_slot; null:
+                            // no block is skipped)
   const float *sdist;       // n: d(s, Rs) in the same order
   const int32_t *sidx;      // n: original reference row
   const int32_t *soff;      // Rs + 1 cluster offsets
@@ -118,6 +123,19 @@ int launch_bounds_filter(const float *drr, int Rq, int Rs, const float *qrad,
                          const float *sdist, const float *scmax, int k, int d,
                          float *theta0, int32_t *rlist, int32_t *rlen,
                          float2 *clb, cudaStream_t s);
+// Block order of narrow rows (at most 8 floats): within every cluster the
+// rows that lie near one another become neighbours in `out` (the sorted
+// position -> row map that perm holds by distance; out may be perm).
+bool narrow_rows(int dp4);
+int launch_block_order(const float4 *rows, int dp4, int d, const float4 *reps,
+                       const uint64_t *skeys, const int32_t *off, const int32_t *perm, int64_t n,
+                       int32_t *out, cudaStream_t s);
+// Bounding boxes of the blocks of 32 rows of every cluster: block_count(n, R)
+// slots of 2 dp4 float4, block j of cluster c at block_slot(off[c], c) + j.
+__host__ __device__ inline int64_t block_slot(int64_t first, int c) { return first / 32 + c; }
+inline int64_t block_count(int64_t n, int R) { return n / 32 + R + 1; }
+int launch_block_boxes(const float4 *srows, int dp4, int d, const uint64_t *skeys,
+                       const int32_t *off, int64_t n, float4 *boxes, cudaStream_t s);
 int launch_scan(const ScanArgs &a, int num_sms, cudaStream_t s);
 
 // Arguments of the BF16 tensor-core tile search with FP32 re-ranking

@@ -308,8 +308,21 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   const float4 *Rp = nullptr, *Qp = nullptr;
   rc = cluster_side(p, p.S, r, n, p.Rs, &Rp, s);
   if (rc != KNN_OK) return rc;
+  // narrow rows: the block order in place of the order by distance, the boxes
+  // in the sort's input keys (no longer needed) where they fit: without them
+  // the scan skips whole clusters only
+  const bool narrow = narrow_rows(p.tmpl);
+  float4 *boxes = nullptr;
+  if (narrow) {
+    if ((uint64_t)block_count(n, p.Rs) * 2 * p.dp4s * sizeof(float4) <= (uint64_t)n * 8)
+      boxes = reinterpret_cast<float4 *>(p.S.keys);
+    rc = launch_block_order(Rp, p.dp4s, d, p.S.reps, p.S.skeys, p.S.off, p.S.perm, n, p.S.perm, s);
+    if (rc != KNN_OK) return rc;
+  }
   rc = launch_cluster_layout(p.S.skeys, p.S.perm, n, Rp, p.dp4s, p.idx_in_row, p.srows,
                              p.sdist, p.sidx, s);
+  if (rc == KNN_OK && boxes)
+    rc = launch_block_boxes(p.srows, p.dp4s, d, p.S.skeys, p.S.off, n, boxes, s);
   if (rc == KNN_OK) rc = launch_cluster_minmax(p.S.off, p.sdist, p.Rs, p.cmin, p.cmax, s);
   if (rc != KNN_OK) return rc;
   const SideBufs &Qb = p.share ? p.S : p.Q;
@@ -317,6 +330,9 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
     Qp = Rp;
   } else {
     rc = cluster_side(p, p.Q, q, m, p.Rq, &Qp, s);
+    if (rc == KNN_OK && narrow)
+      rc = launch_block_order(Qp, p.dp4s, d, p.Q.reps, p.Q.skeys, p.Q.off, p.Q.perm, m, p.Q.perm,
+                              s);
     if (rc != KNN_OK) return rc;
   }
   rc = launch_query_clusters(Qb.skeys, Qb.off, m, p.Rq, p.qrad, p.slot_cl, s);
@@ -328,6 +344,8 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   ScanArgs a{};
   a.qrows = Qp;
   a.qorder = Qb.perm;
+  a.qreps = Qb.reps;
+  a.boxes = boxes;
   a.slot_cl = p.slot_cl;
   a.qoff = Qb.off;
   a.m = m;

@@ -108,6 +108,10 @@ struct RefSide {
   ClusterSet sset;
   const float4 *Rp = nullptr;  // packed rows, original order
   float4 *srows = nullptr;     // cluster-contiguous rows
+  // narrow rows: slot -> row in block order (the order of srows and sidx; sdist
+  // stays by distance) and the blocks' bounding boxes; null otherwise
+  int32_t *order = nullptr;
+  float4 *boxes = nullptr;
   float *sdist = nullptr, *cmin = nullptr, *cmax = nullptr;
   int32_t *sidx = nullptr;
   int *inexact = nullptr;      // device flag: 0 when the rows are small integers
@@ -120,6 +124,7 @@ struct QuerySide {
   int Rq = 0;
   const float4 *Qp = nullptr;  // query rows (packed), original order
   ClusterSet qset;             // qset.perm: slot -> query row; qset.off: slots of a cluster
+  const int32_t *order = nullptr;  // slot -> query row as the scans take it
   const int *inexact = nullptr;
   float *qrad = nullptr, *drr = nullptr, *theta0 = nullptr;
   int32_t *slot_cl = nullptr, *rlist = nullptr, *rlen = nullptr;

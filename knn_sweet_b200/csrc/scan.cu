@@ -399,14 +399,57 @@ __device__ __forceinline__ bool fp32_exact(const ScanArgs &a) {
 #ifndef KNN_QUERY_THETA0
 #define KNN_QUERY_THETA0 1
 #endif
-__device__ __forceinline__ float query_theta0(const ScanArgs &a, int64_t slot, int qc, float tol) {
+__device__ __forceinline__ float query_theta0(const ScanArgs &a, float dq, int qc, float tol) {
   float th = a.theta0[qc];
-  if (KNN_QUERY_THETA0 && a.qrad && a.qkeys) {
-    const float rq = a.qrad[qc], dq = __uint_as_float((uint32_t)a.qkeys[slot]);
+  if (KNN_QUERY_THETA0 && a.qrad) {
+    const float rq = a.qrad[qc];
     const float cut = (rq - dq) - tol * (rq + dq + th);
     if (cut > 0.0f) th -= cut;
   }
   return th;
+}
+
+// Squared distance of a point to a block's bounding box, in the arithmetic of
+// the distances: every coordinate's gap is at most the difference to any row
+// of the block, and subtraction, squaring and accumulation round
+// monotonically, so no row of the block has a smaller computed distance.  (A
+// difference that is not a number counts as no gap.)
+template <int DP4>
+__device__ __forceinline__ float box_dist2(const float4 (&q)[DP4], const float4 (&lo)[DP4],
+                                           const float4 (&hi)[DP4]) {
+  float acc = 0.0f;
+  auto one = [&](float x, float l, float h) {
+    const float g = fmaxf(fmaxf(__fsub_rn(l, x), __fsub_rn(x, h)), 0.0f);
+    acc = __fmaf_rn(g, g, acc);
+  };
+#pragma unroll
+  for (int c = 0; c < DP4; c++) {
+    one(q[c].x, lo[c].x, hi[c].x);
+    one(q[c].y, lo[c].y, hi[c].y);
+    one(q[c].z, lo[c].z, hi[c].z);
+    one(q[c].w, lo[c].w, hi[c].w);
+  }
+  return acc;
+}
+
+// The same between two boxes: no point of one is nearer to a point of the
+// other.
+template <int DP4>
+__device__ __forceinline__ float boxes_dist2(const float4 (&alo)[DP4], const float4 (&ahi)[DP4],
+                                             const float4 (&blo)[DP4], const float4 (&bhi)[DP4]) {
+  float acc = 0.0f;
+  auto one = [&](float al, float ah, float bl, float bh) {
+    const float g = fmaxf(fmaxf(__fsub_rn(bl, ah), __fsub_rn(al, bh)), 0.0f);
+    acc = __fmaf_rn(g, g, acc);
+  };
+#pragma unroll
+  for (int c = 0; c < DP4; c++) {
+    one(alo[c].x, ahi[c].x, blo[c].x, bhi[c].x);
+    one(alo[c].y, ahi[c].y, blo[c].y, bhi[c].y);
+    one(alo[c].z, ahi[c].z, blo[c].z, bhi[c].z);
+    one(alo[c].w, ahi[c].w, blo[c].w, bhi[c].w);
+  }
+  return acc;
 }
 
 // FP64 re-decision of one query's k-th boundary, by one warp.  s[0..n) holds
@@ -577,12 +620,6 @@ struct QueryRow<0, IDXROW> {
 #ifndef KNN_TARGET_WARPS_WIDE
 #define KNN_TARGET_WARPS_WIDE 16
 #endif
-// Load a small member row together with its band distance (before the band
-// test) so both loads are in flight at once.
-#ifndef KNN_EAGER_ROWS
-#define KNN_EAGER_ROWS 1
-#endif
-
 // Traversal choices (compile-time): visit a chunk's clusters nearest d(q,Rs)
 // first, and walk each band outward from d(s,Rs) ~ d(q,Rs).
 #ifndef KNN_ORDER_BY_D
@@ -642,8 +679,8 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
   const float tol = bound_tol(a.d);
   unsigned evals = 0;
   constexpr bool kWideRows = DP4 == 0 || DP4 >= 4;
-  // small rows: load the member row together with its band distance
-  constexpr bool kEagerRow = KNN_EAGER_ROWS && (DP4 > 0 && DP4 <= 2);
+  // narrow rows: members in block order, blocks of 32 skipped by their boxes
+  constexpr bool kBlocks = DP4 == 1 || DP4 == 2;
   // statistics: per-lane 32-bit counts folded once per query into per-block
   // shared counters, added to the global ones at exit
   __shared__ unsigned long long blk_ctr[kScanCounters];
@@ -676,7 +713,12 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
 #endif
     QueryRow<DP4, IDXROW> qr;
     qr.load(a.qrows, q, dp4, qslot);
-    tk.reset(query_theta0(a, slot, qc, tol), lane);
+    // the query's distance to its representative: slots of narrow rows are in
+    // block order, so it is computed; others carry it in their sort key
+    float dq = __int_as_float(0x7f800000);
+    if constexpr (kBlocks) dq = sqrtf(qr.dist2(a.qreps + (int64_t)qc * DP4, DP4));
+    else if (a.qkeys) dq = __uint_as_float((uint32_t)a.qkeys[slot]);
+    tk.reset(query_theta0(a, dq, qc, tol), lane);
 
     // one band step: lane's member p of the cluster at `start`, kept when
     // its distance to the representative lies in [lo_v, hi_v]
@@ -691,16 +733,14 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       float dsv = 0.0f, v = 0.0f;
       int32_t idx = 0;
       bool inb;
-      if constexpr (kEagerRow) {
-        // small rows: issue the row load together with the band distance
-        float4 row[DP4];
-        if (valid) {
+      if constexpr (kBlocks) {
+        inb = valid;
+        if (inb) {
+          float4 row[DP4];
 #pragma unroll
           for (int c = 0; c < DP4; c++) row[c] = a.srows[(size_t)gp * DP4 + c];
-          dsv = a.sdist[gp];
+          v = qr.dist2_member(row, &idx);
         }
-        inb = valid && dsv >= lo_v && dsv <= hi_v;
-        if (inb) v = qr.dist2_member(row, &idx);
       } else if constexpr (DP4 > 0) {
         dsv = valid ? a.sdist[gp] : 0.0f;
         inb = valid && dsv >= lo_v && dsv <= hi_v;
@@ -848,6 +888,35 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const int start = a.soff[c];
         const int n_c = a.soff[c + 1] - start;
 #endif
+        if constexpr (kBlocks) {
+          // a lane per block of 32 members: the blocks whose box comes within
+          // the threshold, in order, as long as they still do
+          const int nblk = (n_c + 31) >> 5;
+          const int64_t slot0 =
+              a.boxes ? block_slot(start, __shfl_sync(kFull, rs, src)) : 0;
+          for (int b0 = 0; b0 < nblk; b0 += 32) {
+            float bd = b0 + lane < nblk ? 0.0f : __int_as_float(0x7f800000);
+            if (a.boxes && b0 + lane < nblk) {
+              float4 lo[DP4], hi[DP4];
+              const float4 *b = a.boxes + (slot0 + b0 + lane) * 2 * DP4;
+#pragma unroll
+              for (int e = 0; e < DP4; e++) {
+                lo[e] = b[e];
+                hi[e] = b[DP4 + e];
+              }
+              bd = box_dist2<DP4>(qr.v, lo, hi);
+            }
+            unsigned todo = __ballot_sync(kFull, b0 + lane < nblk && !(bd > tk.thr_d2));
+            while (todo) {
+              const int t = __ffs((int)todo) - 1;
+              todo &= todo - 1;
+              if (__shfl_sync(kFull, bd, t) > tk.thr_d2) continue;
+              const int p = 32 * (b0 + t) + lane;
+              step(start, p, p < n_c, 0.0f, 0.0f);
+            }
+          }
+          continue;
+        }
 #if KNN_WALK_OUTWARD
         // members below `mid` have d(s,Rs) < Dc, from `mid` on >= Dc; walk
         // outward from there, alternately up and down
@@ -970,12 +1039,12 @@ static int launch_scan_l(const ScanArgs &a, int num_sms, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Group scan for small k (k <= 32) and narrow rows (d <= 8): one warp, up to
 // 32 queries of one query cluster, a query per lane.  The queries share their
-// cluster's candidate list, so the warp walks it once for all of them: every
-// reference cluster that some lane still needs (the scan's own two tests, per
-// lane) contributes the members in the union of those lanes' bands
-// |D - d(s,Rs)| <= theta, 32 at a time through shared memory, and every lane
-// evaluates the same member in the same instruction -- coalesced row loads,
-// broadcast shared-memory reads, no divergence between lanes.
+// cluster's candidate list, so the warp walks it once for all of them: a lane
+// tests one listed cluster (or one block of 32 members) against the queries'
+// bounding box and largest threshold, the blocks left come nearest first, and
+// a block that some lane's own threshold reaches goes through shared memory:
+// every lane evaluates the same member in the same instruction -- coalesced
+// row loads, broadcast shared-memory reads, no divergence between lanes.
 //
 // A candidate (d^2 at most the lane's threshold) goes into the lane's column
 // of a shared-memory buffer; when some lane's column is nearly full, all lanes
@@ -984,12 +1053,13 @@ static int launch_scan_l(const ScanArgs &a, int num_sms, cudaStream_t s) {
 // lane's threshold.
 //
 // What bounds it: instruction issue (75 % of the slots on 512 surface clouds,
-// k = 16) and the ALU pipe of the merges.  It replaced a thread per query whose
-// every insertion into a sorted list of 64-bit keys was executed by the whole
-// warp: 4,096 surface clouds, k = 16: search 59.4 -> 22.4 ms; 64 pairs of
-// clouds, k = 8 both ways: 3.2 -> 1.4 ms.  64-bit keys in the merges instead
-// of distance words: 32 ms; three blocks per SM (111 registers): 24.2 ms, six
-// (80 registers, spilling): 28 ms.
+// k = 16), about half of it the members and a third the merges (13 blocks and
+// 7.7 merges per group).  It replaced a thread per query whose every insertion
+// into a sorted list of 64-bit keys was executed by the whole warp: 4,096
+// surface clouds, k = 16: search 59.4 -> 20.4 ms.  64-bit keys in the merges
+// instead of distance words: 32 ms; whole clusters by their distance band
+// instead of blocks by their boxes: 22.4 ms; candidates stored by predicated
+// instructions instead of a branch: 22.4 ms.
 //
 // FP64 boundary: the threshold is band_hi of the k-th key, so every point
 // inside the final k-th's FP32 band is evaluated and admitted; one that a merge
@@ -1166,8 +1236,6 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
   // the current 32 members by coordinate (negated); the last pad coordinate
   // of rows that carry their index there is the index
   __shared__ __align__(16) float s_mem[kGroupWarps][4 * DP4 + (IDXROW ? 0 : 1)][32];
-  __shared__ float4 s_rep[kGroupWarps][32 * DP4];  // representatives of the list batch
-  __shared__ float4 s_meta[kGroupWarps][32];       // their cmax, cmin, start, size
   __shared__ unsigned long long blk_ctr[4];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x < 4) blk_ctr[threadIdx.x] = 0;
@@ -1179,7 +1247,7 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
   const int64_t nslots = a.slot_list ? (int64_t)*a.slot_count : a.m;
   TK tk;
   tk.col = &s_col[w][K > 1 ? lane : 0];
-  unsigned evals = 0, visited = 0, pruned = 0, pushed = 0;
+  unsigned evals = 0, visited = 0, listed = 0, pushed = 0;
 
   // Windows of 32 slots from the work counter.  Without a slot list a window
   // stands for the groups that start in it (they begin at every 32nd slot of
@@ -1240,59 +1308,112 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
     }
     tk.reset();
     uint64_t best = kLaneEmpty;  // the list for k = 1
-    float theta = act ? query_theta0(a, slot, qc, tol) : 0.0f;
-    float thr = theta * theta;  // admits every d^2 <= theta0^2, whatever the index
+    float thr = 0.0f;  // squared distances up to it enter
+    if (act) {
+      const float th =
+          query_theta0(a, sqrtf(qr.dist2(a.qreps + (int64_t)qc * DP4, DP4)), qc, tol);
+      thr = th * th;  // admits every d^2 <= theta0^2, whatever the index
+    }
+    // the queries' bounding box (the coordinates behind kCoords are padding)
+    // and the largest threshold among them
+    float4 glo[DP4], ghi[DP4];
+    {
+      float lo[4 * DP4], hi[4 * DP4];
+#pragma unroll
+      for (int c = 0; c < 4 * DP4; c++) {
+        lo[c] = act ? qq[c].x : inf;
+        hi[c] = act ? qq[c].x : -inf;
+        if (c >= kCoords) lo[c] = hi[c] = 0.0f;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int c = 0; c < kCoords; c++) {
+          lo[c] = fminf(lo[c], __shfl_xor_sync(kFull, lo[c], o));
+          hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], o));
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < DP4; e++) {
+        glo[e] = make_float4(lo[4 * e], lo[4 * e + 1], lo[4 * e + 2], lo[4 * e + 3]);
+        ghi[e] = make_float4(hi[4 * e], hi[4 * e + 1], hi[4 * e + 2], hi[4 * e + 3]);
+      }
+    }
+    auto largest = [&](float x) {  // x >= 0 (a NaN counts as the largest)
+      return __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(x)));
+    };
+    float thr_max = largest(thr);
     const int nr = a.rlen[qc];
     const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
     for (int base = 0; base < nr; base += 32) {
-      const int nb = min(32, nr - base);
-      __syncwarp();
-      if (lane < nb) {
-        const int c = rl[base + lane];
+      // a lane per reference cluster: it can hold a member within some
+      // query's threshold only if the queries' box comes within theta +
+      // radius of its representative
+      int c = 0, cst = 0, cnn = 0;
+      float need_th = inf;  // the smallest theta that needs the cluster
+      if (base + lane < nr) {
+        c = rl[base + lane];
+        float4 rep[DP4];
 #pragma unroll
-        for (int e = 0; e < DP4; e++) s_rep[w][lane * DP4 + e] = a.sreps[(int64_t)c * DP4 + e];
-        const int st = a.soff[c];
-        s_meta[w][lane] = make_float4(a.cmax[c], a.cmin[c], __int_as_float(st),
-                                      __int_as_float(a.soff[c + 1] - st));
+        for (int e = 0; e < DP4; e++) rep[e] = a.sreps[(int64_t)c * DP4 + e];
+        const float Dg = sqrtf(box_dist2<DP4>(rep, glo, ghi));
+        cst = a.soff[c];
+        cnn = a.soff[c + 1] - cst;
+        // D - cmax > theta + tol (2 D + 2 theta), solved for theta
+        if (cnn > 0) need_th = (Dg - 2.0f * tol * Dg - a.cmax[c]) * (1.0f - 2.0f * tol);
       }
-      __syncwarp();
-      for (int i = 0; i < nb; i++) {
-        const float D = sqrtf(qr.dist2(&s_rep[w][i * DP4], DP4));
-        const float4 mt = s_meta[w][i];
-        float slack = tol * (2.0f * D + 2.0f * theta);
-        const bool need = act && !(D - mt.x > theta + slack || D + theta + slack < mt.y);
-        visited += need;
-        pruned += act && !need;
-        if (!__any_sync(kFull, need)) continue;
-        // the union of the lanes' bands; a NaN edge (a lane whose distances
-        // are not numbers) opens the band instead of closing it
-        const float lo_l = D - theta - slack, hi_l = D + theta + slack;
-        const float lo = __uint_as_float(__reduce_min_sync(
-            kFull, __float_as_uint(need ? fmaxf(lo_l, 0.0f) : inf)));
-        const float hi = __uint_as_float(__reduce_max_sync(
-            kFull, __float_as_uint(need ? (hi_l < inf ? fmaxf(hi_l, 0.0f) : inf) : 0.0f)));
-        float cut = need ? thr : -1.0f;  // no d^2 passes a lane that is done with c
-        const int start = __float_as_int(mt.z), n_c = __float_as_int(mt.w);
-        for (int c0 = 0; c0 < n_c; c0 += 32) {
-          const int p = c0 + lane;
-          const bool valid = p < n_c;
-          const unsigned gp = (unsigned)(start + p);
-          float4 row[DP4];
-          float ds = inf;
-          if (valid) {
-            ds = a.sdist[gp];
+      unsigned clusters = __ballot_sync(kFull, !(need_th > sqrtf(thr_max)));
+      while (clusters) {
+        const int ci = __ffs((int)clusters) - 1;
+        clusters &= clusters - 1;
+        if (__shfl_sync(kFull, need_th, ci) > sqrtf(thr_max)) continue;
+        const int start = __shfl_sync(kFull, cst, ci), n_c = __shfl_sync(kFull, cnn, ci);
+        const int64_t slot0 = a.boxes ? block_slot(start, __shfl_sync(kFull, c, ci)) : 0;
+        const int nblk = (n_c + 31) >> 5;
+        bool hit = false;
+        for (int b0 = 0; b0 < nblk; b0 += 32) {
+          // a lane per block of 32 members, nearest the queries' box first
+          uint32_t bd = b0 + lane < nblk ? 0u : 0xffffffffu;
+          if (a.boxes && b0 + lane < nblk) {
+            const float4 *b = a.boxes + (slot0 + b0 + lane) * 2 * DP4;
+            float4 gap_lo[DP4], gap_hi[DP4];
 #pragma unroll
-            for (int e = 0; e < DP4; e++) row[e] = a.srows[(size_t)gp * DP4 + e];
-          } else {
-            // a row that passes no lane: its distances are NaN
+            for (int e = 0; e < DP4; e++) {
+              gap_lo[e] = b[e];
+              gap_hi[e] = b[DP4 + e];
+            }
+            bd = __float_as_uint(boxes_dist2<DP4>(glo, ghi, gap_lo, gap_hi));
+          }
+          for (;;) {
+            const uint32_t nearest = __reduce_min_sync(kFull, bd);
+            if (nearest == 0xffffffffu || __uint_as_float(nearest) > thr_max) break;
+            const int bi = __ffs((int)__ballot_sync(kFull, bd == nearest)) - 1;
+            if (lane == bi) bd = 0xffffffffu;
+            const int p = 32 * (b0 + bi) + lane;
+            const bool valid = p < n_c;
+            const unsigned gp = (unsigned)(start + p);
+            float4 row[DP4];
 #pragma unroll
             for (int e = 0; e < DP4; e++)
-              row[e] = make_float4(__int_as_float(0x7fffffff), 0.0f, 0.0f, 0.0f);
-          }
-          const bool inb = valid && ds >= lo && !(ds > hi);
-          const unsigned bm = __ballot_sync(kFull, inb);
-          const bool last = __ballot_sync(kFull, valid && !(ds > hi)) != kFull;
-          if (bm) {
+              // (a row past the end passes no lane: its distances are NaN)
+              row[e] = valid ? a.srows[(size_t)gp * DP4 + e]
+                             : make_float4(__int_as_float(0x7fffffff), 0.0f, 0.0f, 0.0f);
+            bool need = act;
+            if (a.boxes) {
+              const float4 *b = a.boxes + (slot0 + b0 + bi) * 2 * DP4;
+              float4 lo[DP4], hi[DP4];
+#pragma unroll
+              for (int e = 0; e < DP4; e++) {
+                lo[e] = b[e];
+                hi[e] = b[DP4 + e];
+              }
+              need = act && !(box_dist2<DP4>(qr.v, lo, hi) > thr);
+            }
+            if (!__any_sync(kFull, need)) continue;
+            hit |= need;
+            const int cnt = min(32, n_c - 32 * (b0 + bi));
+            if (need) evals += (unsigned)cnt;
+            float cut = need ? thr : -1.0f;  // no d^2 passes a lane that does not need the block
             __syncwarp();
 #pragma unroll
             for (int e = 0; e < DP4; e++) {
@@ -1304,11 +1425,8 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
             if constexpr (!IDXROW)
               s_mem[w][4 * DP4][lane] = valid ? __int_as_float(a.sidx[gp]) : 0.0f;
             __syncwarp();
-            const int p1 = 31 - __clz((int)bm);
-            const int p0 = (__ffs((int)bm) - 1) & ~3;
-            // four members at a time (the few outside the band that this
-            // rounds in are members too: their distances are as good)
-            for (int t = p0; t <= p1; t += 4) {
+            bool tightened = K == 1;  // warp-uniform
+            for (int t = 0; t < cnt; t += 4) {
               // packed FP32 pairs, the scan's arithmetic for each member
               float2 v01, v23;
 #pragma unroll
@@ -1341,26 +1459,29 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
                   pushed += tk.cnt - tk.kept;
                   tk.flush(k, d, thr);
                   if (need) cut = thr;
+                  tightened = true;
                 }
               } else if (best != kLaneEmpty) {
                 thr = band_hi(key_d2(best), d);
                 if (need) cut = thr;
               }
             }
-            if (need) evals += (unsigned)(p1 - p0 + 1);
+            if (tightened) thr_max = largest(thr);
           }
-          if (last) break;
         }
-        theta = fminf(theta, sqrtf(thr));
+        visited += hit;
       }
     }
-    // the K best keys, ascending
-    uint64_t key[K];
+    if (act) listed += nr;
     if constexpr (K > 1) {
       if (__any_sync(kFull, tk.cnt > tk.kept)) {
         pushed += tk.cnt - tk.kept;
         tk.flush(k, d, thr);
       }
+    }
+    // the K best keys, ascending
+    uint64_t key[K];
+    if constexpr (K > 1) {
       if (__any_sync(kFull, tk.kept > K)) tk.cut();
 #pragma unroll
       for (int j = 0; j < K; j++) {
@@ -1439,6 +1560,7 @@ __global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 :
     }
   }
   if (a.counters) {
+    unsigned pruned = listed - visited;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       evals += __shfl_xor_sync(kFull, evals, o);
@@ -1557,8 +1679,11 @@ __global__ void __launch_bounds__(kBandThreads) band_resolve_kernel(const ScanAr
   extern __shared__ __align__(16) unsigned char smem_raw[];
   BandEntry *ent = reinterpret_cast<BandEntry *>(smem_raw);
   float *qv = reinterpret_cast<float *>(ent + kBandCap);  // 4 * dp4 floats
-  __shared__ int s_cnt;
+  __shared__ int s_cnt, s_nvis;
   __shared__ BandEntry s_thr;
+  __shared__ int s_vis[kBandThreads];
+  __shared__ float s_D[kBandThreads];
+  const bool narrow = a.dp4_tmpl == 1 || a.dp4_tmpl == 2;
   const int tid = threadIdx.x, k = a.k, d = a.d, dp4 = a.dp4;
   const float tol = bound_tol(d);
   const unsigned total = *a.unres_count;
@@ -1583,43 +1708,86 @@ __global__ void __launch_bounds__(kBandThreads) band_resolve_kernel(const ScanAr
     __syncthreads();
     const int nr = a.rlen[qc];
     const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
-    for (int j = 0; j < nr; j++) {  // block-uniform
-      const int c = rl[j];
-      const float D =
-          sqrtf(band_dist2(qv, reinterpret_cast<const float *>(a.sreps + (int64_t)c * dp4), d));
-      const float slack = tol * (2.0f * D + 2.0f * th);
-      if (D - a.cmax[c] > th + slack || D + th + slack < a.cmin[c]) continue;
-      const int start = a.soff[c], n_c = a.soff[c + 1] - start;
-      const float lo_e = D - th - slack, hi_e = D + th + slack;
-      int p0 = 0, p1 = n_c;  // first member with d(s, Rc) >= lo_e
-      while (p0 < p1) {
-        const int md = (p0 + p1) >> 1;
-        if (a.sdist[start + md] < lo_e) p0 = md + 1;
-        else p1 = md;
-      }
-      for (int c0 = p0; c0 < n_c; c0 += kBandThreads) {  // block-uniform
-        const int p = c0 + tid;
-        bool past = p >= n_c;
-        if (!past) {
-          const int64_t gp = (int64_t)start + p;
-          if (a.sdist[gp] > hi_e) {
-            past = true;
-          } else {
-            const float v =
-                band_dist2(qv, reinterpret_cast<const float *>(a.srows + gp * dp4), d);
-            if (v >= lo && v <= hi) {
-              const int32_t id = a.sidx[gp];
-              const double w =
-                  dist2_f64(qv, reinterpret_cast<const float *>(a.rrows + (int64_t)id * dp4), d);
-              evals++;
-              const BandEntry e{(unsigned long long)__double_as_longlong(w), make_key(v, id)};
-              if (band_entry_less(e, s_thr)) ent[atomicAdd(&s_cnt, 1)] = e;
-            }
+    // one member (a block-uniform number of calls): into the set when its
+    // FP32 distance lies in the band
+    auto member = [&](bool in, int64_t gp) {
+      // the set is full when one of this step's additions made it so: each
+      // thread judges by its own addition's place, so that the decision is
+      // the same for all (the count itself may move on while others read it)
+      int full = 0;
+      if (in) {
+        const float v = band_dist2(qv, reinterpret_cast<const float *>(a.srows + gp * dp4), d);
+        if (v >= lo && v <= hi) {
+          const int32_t id = a.sidx[gp];
+          const double w =
+              dist2_f64(qv, reinterpret_cast<const float *>(a.rrows + (int64_t)id * dp4), d);
+          evals++;
+          const BandEntry e{(unsigned long long)__double_as_longlong(w), make_key(v, id)};
+          if (band_entry_less(e, s_thr)) {
+            const int at = atomicAdd(&s_cnt, 1);
+            ent[at] = e;
+            full = at + 1 > kBandCap - kBandThreads;
           }
         }
-        const int any_past = __syncthreads_or(past);
-        if (s_cnt > kBandCap - kBandThreads) band_cut(ent, &s_cnt, &s_thr, need);
-        if (any_past) break;
+      }
+      if (__syncthreads_or(full)) band_cut(ent, &s_cnt, &s_thr, need);
+    };
+    // a thread per listed cluster, then the block over each cluster left
+    for (int j0 = 0; j0 < nr; j0 += kBandThreads) {
+      __syncthreads();
+      if (tid == 0) s_nvis = 0;
+      __syncthreads();
+      if (j0 + tid < nr) {
+        const int c = rl[j0 + tid];
+        const float D =
+            sqrtf(band_dist2(qv, reinterpret_cast<const float *>(a.sreps + (int64_t)c * dp4), d));
+        const float slack = tol * (2.0f * D + 2.0f * th);
+        if (!(D - a.cmax[c] > th + slack || D + th + slack < a.cmin[c])) {
+          const int v = atomicAdd(&s_nvis, 1);
+          s_vis[v] = c;
+          s_D[v] = D;
+        }
+      }
+      __syncthreads();
+      const int nvis = s_nvis;
+      for (int v = 0; v < nvis; v++) {  // block-uniform
+        const int c = s_vis[v];
+        const int start = a.soff[c], n_c = a.soff[c + 1] - start;
+        if (narrow) {
+          // members in block order: a warp per block of 32, by its box
+          for (int c0 = 0; c0 < n_c; c0 += kBandThreads) {
+            const int p = c0 + tid;
+            bool in = p < n_c;
+            if (in && a.boxes) {
+              const float *b = reinterpret_cast<const float *>(
+                  a.boxes + (block_slot(start, c) + (p >> 5)) * 2 * dp4);
+              float acc = 0.0f;
+              for (int e = 0; e < d; e++) {
+                const float g =
+                    fmaxf(fmaxf(__fsub_rn(b[e], qv[e]), __fsub_rn(qv[e], b[4 * dp4 + e])), 0.0f);
+                acc = __fmaf_rn(g, g, acc);
+              }
+              in = !(acc > hi);
+            }
+            member(in, (int64_t)start + p);
+          }
+          continue;
+        }
+        const float D = s_D[v], slack = tol * (2.0f * D + 2.0f * th);
+        const float lo_e = D - th - slack, hi_e = D + th + slack;
+        int p0 = 0, p1 = n_c;  // first member with d(s, Rc) >= lo_e
+        while (p0 < p1) {
+          const int md = (p0 + p1) >> 1;
+          if (a.sdist[start + md] < lo_e) p0 = md + 1;
+          else p1 = md;
+        }
+        for (int c0 = p0; c0 < n_c; c0 += kBandThreads) {  // block-uniform
+          const int p = c0 + tid;
+          const bool past = p >= n_c || a.sdist[start + p] > hi_e;
+          const int any_past = __syncthreads_or(past);
+          member(!past, (int64_t)start + p);
+          if (any_past) break;
+        }
       }
     }
     band_cut(ent, &s_cnt, &s_thr, need);
@@ -1675,11 +1843,14 @@ int launch_scan(const ScanArgs &a, int num_sms, cudaStream_t s) {
 }
 
 static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
-  // group scan: small k, rows of at most 8 floats, and short bands (at most
-  // 128 points per cluster on average); with longer ones the warp per query
-  // skips more of a cluster than a group of queries can
-  const bool short_bands = a.n_ref > 0 && a.Rs > 0 && a.n_ref <= 128 * (int64_t)a.Rs;
-  if (a.k <= 32 && short_bands && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
+  // group scan: k <= 32, rows of at most 8 floats, and enough queries that
+  // groups of 32 fill the chip -- below that a warp per query has 32 times the
+  // warps in flight.  Self-joins of d = 3 blobs, search in us, group / warp:
+  // k = 16: 10,000 points 139 / 68, 32,000 231 / 193, 50,000 246 / 301,
+  // 100,000 395 / 635, 10^6 2220 / 8271; k = 1: 10,000 61 / 51, 16,000 70 / 74,
+  // 32,000 84 / 137; k = 32: 50,000 301 / 336.
+  const int64_t fill = (int64_t)num_sms * 32 * (a.k == 1 ? 3 : 8);
+  if (a.k <= 32 && a.m >= fill && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
       return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)
                           : launch_group_scan<1, false>(a, num_sms, s);

@@ -114,6 +114,7 @@ int replicate_sides(Arena &ar, int g, int g0, const RefSide &R, const QuerySide 
   KNN_TRY(replicate(ar, g, g0, R.srows, (size_t)n * dp4, s, &R2->srows));
   KNN_TRY(replicate(ar, g, g0, R.sdist, (size_t)n, s, &R2->sdist));
   KNN_TRY(replicate(ar, g, g0, R.sidx, (size_t)n, s, &R2->sidx));
+  KNN_TRY(replicate(ar, g, g0, R.boxes, (size_t)block_count(n, Rs) * 2 * dp4, s, &R2->boxes));
   KNN_TRY(replicate(ar, g, g0, R.cmin, (size_t)Rs, s, &R2->cmin));
   KNN_TRY(replicate(ar, g, g0, R.cmax, (size_t)Rs, s, &R2->cmax));
   KNN_TRY(replicate(ar, g, g0, R.inexact, 1, s, &R2->inexact));
@@ -132,6 +133,14 @@ int replicate_sides(Arena &ar, int g, int g0, const RefSide &R, const QuerySide 
   }
   Q2->qset.R = Rq;
   KNN_TRY(replicate(ar, g, g0, Q.qset.perm, (size_t)m, s, &Q2->qset.perm));
+  Q2->order = Q2->qset.perm;
+  if (Q.order != Q.qset.perm) {
+    int32_t *order;
+    KNN_TRY(replicate(ar, g, g0, Q.order, (size_t)m, s, &order));
+    Q2->order = order;
+  }
+  if (R.boxes)
+    KNN_TRY(replicate(ar, g, g0, Q.qset.reps, (size_t)Rq * dp4, s, &Q2->qset.reps));
   KNN_TRY(replicate(ar, g, g0, Q.qset.off, (size_t)Rq + 1, s, &Q2->qset.off));
   KNN_TRY(replicate(ar, g, g0, Q.slot_cl, (size_t)m, s, &Q2->slot_cl));
   KNN_TRY(replicate(ar, g, g0, Q.theta0, (size_t)Rq, s, &Q2->theta0));

@@ -1,0 +1,72 @@
+"""Joins of narrow rows (d <= 8): the block order of the clusters, the group
+scan (k <= 32 and enough queries) and the warp scan over blocks.
+
+Sizes sit where they can go wrong: clusters of a few members, blocks of 32 and
+runs of 1,024 positions with one row more or less, the smallest and largest k
+of every list length, and crowds of equal distances that overflow a lane's
+candidate column.  Group-scan cases pass at least 38,000 queries.
+"""
+import numpy as np
+import pytest
+
+from knn_sweet_b200 import knnjoin
+from tests.parity import assert_matches
+
+pytestmark = pytest.mark.gpu
+
+MANY = 38_401  # queries: the group scan, with a remainder of one
+
+
+def _check(oracle, q, r, k, exact=False, sample=600, **kw):
+    idx, dist = knnjoin(q, r, k, **kw)
+    rows = np.random.default_rng(1).permutation(q.shape[0])[:sample]
+    oi, od = oracle.bruteforce_f64(q[rows], r, k)
+    assert_matches(idx[rows], dist[rows], oi, od, exact=exact)
+
+
+@pytest.mark.parametrize("d,k", [(1, 1), (2, 4), (3, 1), (3, 2), (3, 5), (3, 8), (3, 9), (3, 16),
+                                 (3, 17), (3, 32), (4, 8), (4, 32), (5, 16), (8, 1), (8, 20)])
+def test_group_scan_float_rows(cuda_device, oracle, d, k):
+    rng = np.random.default_rng(10 * d + k)
+    r = rng.standard_normal((2049, d)).astype(np.float32)
+    q = rng.standard_normal((MANY, d)).astype(np.float32)
+    _check(oracle, q, r, k)
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 32, 33, 1023, 1024, 1025])
+def test_group_scan_reference_sizes(cuda_device, oracle, n):
+    rng = np.random.default_rng(n)
+    r = rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    q = rng.uniform(-1, 1, (MANY, 3)).astype(np.float32)
+    _check(oracle, q, r, 16, sreps=min(n, 7))
+
+
+@pytest.mark.parametrize("k", [1, 4, 16, 31])
+def test_group_scan_crowds_of_equal_distances(cuda_device, oracle, k):
+    # 64 distinct integer points, 600 copies of each: every list overflows with ties
+    rng = np.random.default_rng(k)
+    base = rng.integers(0, 4, (64, 3)).astype(np.float32)
+    x = base[rng.integers(0, 64, MANY)]
+    _check(oracle, x, x, k, exact=True, sample=200)
+    # the same shifted off the integers: the boundary is decided in FP64
+    y = x + np.float32(0.1)
+    _check(oracle, y, y, k, sample=200)
+
+
+@pytest.mark.parametrize("d,k,sreps", [(1, 40, 3), (3, 33, 1), (3, 64, 50), (3, 200, 9),
+                                       (4, 100, 4), (6, 300, 20), (8, 1000, 5), (3, 24, 2)])
+def test_warp_scan_over_blocks(cuda_device, oracle, d, k, sreps):
+    rng = np.random.default_rng(100 * d + k)
+    r = rng.standard_normal((3000, d)).astype(np.float32)
+    q = rng.standard_normal((257, d)).astype(np.float32)
+    _check(oracle, q, r, k, sample=257, sreps=sreps)
+
+
+def test_tiny_clusters_and_far_outliers(cuda_device, oracle):
+    # as many representatives as points, and one point that stretches a cluster
+    rng = np.random.default_rng(5)
+    r = rng.standard_normal((500, 3)).astype(np.float32)
+    r[17] = 1e6
+    q = rng.standard_normal((MANY, 3)).astype(np.float32)
+    _check(oracle, q, r, 8, sreps=500)
+    _check(oracle, q, r, 8, sreps=1, qreps=1)
