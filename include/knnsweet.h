@@ -85,8 +85,9 @@ typedef struct knn_options {
   int32_t flags;      /* KNN_SQUARED_DIST | KNN_NO_TENSOR_CORES, or 0        */
   int32_t lloyd_iters;/* representative refinement: after the draw, this many
                          steps of "move every representative to its cluster's
-                         centroid, re-assign" (0 = the reference's draw only;
-                         default 0)                                          */
+                         centroid, re-assign", on a sample of the rows where
+                         there are many per representative (0 = the
+                         reference's draw only; default 0)                   */
   int32_t reserved0;
 } knn_options;
 

@@ -182,6 +182,9 @@ int default_reps(int64_t n) {
 }
 
 
+// Rows per representative that a refinement step looks at.
+constexpr int kLloydPerRep = 16;
+
 int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d, int dp4s, int R,
                    uint32_t seed, int trials, int lloyd_iters, bool use_tc, int *err,
                    cudaStream_t s, ClusterSet *cs) {
@@ -218,22 +221,45 @@ int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d,
   KNN_TRY(keep.alloc(&cs->off, (size_t)R + 1));
   // nearest representative (BF16 tensor-core arg-min + exact FP32 distance to
   // the winner for d >= 16, FP32 CUDA cores otherwise), then one sort into
-  // clusters; with Lloyd steps the representatives move to their clusters'
-  // centroids (the smallest clusters' representatives to the farthest member
-  // of the widest clusters) and the points are assigned and sorted again
-  for (int it = 0; it <= lloyd_iters; it++) {
-    if (it > 0) {
-      KNN_TRY(launch_centroids(rows, dp4s, cs->perm, cs->off, R, cs->reps, s));
-      KNN_TRY(launch_split_clusters(rows, dp4s, cs->perm, cs->off, cs->skeys, R, cs->reps, s));
-    }
+  // clusters
+  auto cluster = [&](const float4 *x, int64_t cnt) -> int {
     if (tc_assign)
-      KNN_TRY(launch_assign_tc(rows, n, dp4s, d, cs->reps, R, tc_scratch, cl, dr, err, s));
+      KNN_TRY(launch_assign_tc(x, cnt, dp4s, d, cs->reps, R, tc_scratch, cl, dr, err, s));
     else
-      KNN_TRY(launch_assign(rows, n, dp4s, cs->reps, R, cl, dr, s));
-    KNN_TRY(launch_cluster_sort(cl, dr, n, R, keys, vals, cs->skeys, cs->perm, temp,
+      KNN_TRY(launch_assign(x, cnt, dp4s, cs->reps, R, cl, dr, s));
+    KNN_TRY(launch_cluster_sort(cl, dr, cnt, R, keys, vals, cs->skeys, cs->perm, temp,
                                 temp_bytes, s));
-    KNN_TRY(launch_cluster_offsets(cs->skeys, n, R, cs->off, s));
+    return launch_cluster_offsets(cs->skeys, cnt, R, cs->off, s);
+  };
+  // Lloyd steps: the representatives move to their clusters' centroids (the
+  // smallest clusters' representatives to the farthest member of the widest
+  // clusters) and the points are assigned and sorted again.  They run on a
+  // sample of about kLloydPerRep rows per representative -- a centroid of that
+  // many is as good a centre, and the clusters only steer the pruning -- and
+  // every row is assigned once, at the end.  Steps over all rows / 100 / 48 /
+  // 24 / 16 rows per representative, whole BF16 joins in ms: N = 2,000,000,
+  // d = 128, 8,192 representatives, 4 steps 44.0 / 33.8 / 27.9 / 25.4 / 24.2
+  // (build 34.4 / 24.3 / 18.3 / 16.2 / 15.5, search 9.4 / 9.4 / 9.6 / 9.1 /
+  // 8.7); N = 1,000,000, d = 32, 1,000 representatives, 3 steps 8.7 / 6.1 / 6.0
+  // / 6.0 / 5.8.
+  if (lloyd_iters > 0) {
+    const int64_t stride = n / ((int64_t)R * kLloydPerRep);
+    const float4 *x = rows;
+    int64_t cnt = n;
+    if (stride > 1) {
+      float4 *sample;
+      cnt = n / stride;
+      KNN_TRY(ar.alloc(&sample, (size_t)cnt * dp4s));
+      KNN_TRY(launch_sample_rows(rows, dp4s, stride, cnt, seed, sample, s));
+      x = sample;
+    }
+    for (int it = 0; it < lloyd_iters; it++) {
+      KNN_TRY(cluster(x, cnt));
+      KNN_TRY(launch_centroids(x, dp4s, cs->perm, cs->off, R, cs->reps, s));
+      KNN_TRY(launch_split_clusters(x, dp4s, cs->perm, cs->off, cs->skeys, R, cs->reps, s));
+    }
   }
+  KNN_TRY(cluster(rows, n));
   return KNN_OK;
 }
 

@@ -794,6 +794,29 @@ int launch_exact_check(const float *x, int64_t count, int d, int *inexact, cudaS
   return KNN_OK;
 }
 
+__global__ void sample_rows_kernel(const float4 *__restrict__ rows, int dp4, int64_t stride,
+                                   int64_t cnt, uint32_t seed, float4 *__restrict__ out) {
+  const int64_t total = cnt * dp4;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = t / dp4;
+    uint32_t h = (uint32_t)i * 0x9e3779b1u + seed;
+    h ^= h >> 15;
+    h *= 0x85ebca77u;
+    h ^= h >> 13;
+    const int64_t src = i * stride + (int64_t)(h % (uint32_t)stride);
+    out[t] = rows[src * dp4 + (t - i * dp4)];
+  }
+}
+
+int launch_sample_rows(const float4 *rows, int dp4, int64_t stride, int64_t cnt, uint32_t seed,
+                       float4 *out, cudaStream_t s) {
+  if (cnt == 0) return KNN_OK;
+  sample_rows_kernel<<<grid_for(cnt * dp4, 256), 256, 0, s>>>(rows, dp4, stride, cnt, seed, out);
+  KNN_LAUNCH_CHECK();
+  return KNN_OK;
+}
+
 int launch_pack_rows(const float *src, int64_t n, int d, int dp4, float4 *dst,
                      cudaStream_t s) {
   if (n == 0) return KNN_OK;

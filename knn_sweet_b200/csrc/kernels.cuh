@@ -94,6 +94,10 @@ size_t assign_tc_scratch_bytes(int R, int d);
 int launch_assign_tc(const float4 *rows, int64_t n, int dp4, int d, const float4 *reps, int R,
                      void *scratch, int32_t *cl, float *dr, int *err, cudaStream_t s);
 size_t cluster_sort_temp_bytes(int64_t n, int R);
+// Row i of `out`: one of rows i * stride .. i * stride + stride - 1, picked by a
+// hash of (seed, i), so that no period of the data is sampled in step.
+int launch_sample_rows(const float4 *rows, int dp4, int64_t stride, int64_t cnt, uint32_t seed,
+                       float4 *out, cudaStream_t s);
 int launch_centroids(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off, int R,
                      float4 *reps, cudaStream_t s);
 int launch_split_clusters(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off,
