@@ -340,13 +340,14 @@ int build_ref_side(Arena &keep, Arena &tmp, const float *r, int64_t n, int d, in
   const bool use_tc = (o.flags & KNN_NO_TENSOR_CORES) == 0;
   KNN_TRY(build_clusters(keep, tmp, R->Rp, n, d, dp4s, Rs, o.seed, o.rep_trials, o.lloyd_iters,
                          use_tc, dev_err, s, &R->sset));
-  KNN_TRY(keep.alloc(&R->srows, (size_t)n * dp4s));
+  R->col_blocks = !narrow_rows(R->tmpl);
+  KNN_TRY(keep.alloc(&R->srows, (size_t)srows_count(n, dp4s, R->col_blocks)));
   KNN_TRY(keep.alloc(&R->sdist, (size_t)n));
   KNN_TRY(keep.alloc(&R->sidx, (size_t)n));
   KNN_TRY(keep.alloc(&R->cmin, (size_t)Rs));
   KNN_TRY(keep.alloc(&R->cmax, (size_t)Rs));
-  // rows with a spare pad float carry their index there (register-width rows)
-  R->idx_in_row = R->tmpl > 0 && 4 * dp4s > d;
+  // narrow rows with a spare pad float carry their index there
+  R->idx_in_row = narrow_rows(R->tmpl) && 4 * dp4s > d;
   const int32_t *order = R->sset.perm;
   if (narrow_rows(R->tmpl)) {
     KNN_TRY(keep.alloc(&R->order, (size_t)n));
@@ -355,8 +356,8 @@ int build_ref_side(Arena &keep, Arena &tmp, const float *r, int64_t n, int d, in
                                R->sset.perm, n, R->order, s));
     order = R->order;
   }
-  KNN_TRY(launch_cluster_layout(R->sset.skeys, order, n, R->Rp, dp4s, R->idx_in_row, R->srows,
-                                R->sdist, R->sidx, s));
+  KNN_TRY(launch_cluster_layout(R->sset.skeys, order, n, R->Rp, dp4s, R->idx_in_row,
+                                R->col_blocks, R->srows, R->sdist, R->sidx, s));
   if (R->boxes)
     KNN_TRY(launch_block_boxes(R->srows, dp4s, d, R->sset.skeys, R->sset.off, n, R->boxes, s));
   KNN_TRY(launch_cluster_minmax(R->sset.off, R->sdist, Rs, R->cmin, R->cmax, s));
@@ -465,8 +466,9 @@ int build_query_side(const RefSide &R, bool share, const float *q, int64_t m, in
   KNN_TRY(ar.alloc(&Q->rlist, (size_t)Rq * Rs));
   KNN_TRY(ar.alloc(&Q->rlen, (size_t)Rq));
   KNN_TRY(ar.alloc(&Q->clb, (size_t)Rq * ((Rs + 31) / 32)));
+  KNN_TRY(ar.alloc(&Q->rlb, (size_t)Rq * Rs));
   KNN_TRY(launch_bounds_filter(Q->drr, Rq, Rs, Q->qrad, Q->qset.off, R.sset.off, R.sdist, R.cmax,
-                               k, d, Q->theta0, Q->rlist, Q->rlen, Q->clb, s));
+                               k, d, Q->theta0, Q->rlist, Q->rlen, Q->clb, Q->rlb, s));
   return KNN_OK;
 }
 
@@ -553,6 +555,8 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   a.qorder = Q.order;
   a.qreps = Q.qset.reps;
   a.boxes = R.boxes;
+  a.col_blocks = R.col_blocks;
+  a.rlb = Q.rlb;
   a.slot_cl = Q.slot_cl;
   a.qoff = Q.qset.off;
   a.m = nslot;

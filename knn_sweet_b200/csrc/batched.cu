@@ -488,14 +488,15 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       float4 *srows;
       float *sdist, *cmin, *cmax;
       int32_t *sidx;
-      KNN_TRY(ar.alloc(&srows, (size_t)n * dp4));
+      const bool cols = !narrow_rows(dp4);
+      KNN_TRY(ar.alloc(&srows, (size_t)srows_count(n, dp4, cols)));
       KNN_TRY(ar.alloc(&sdist, (size_t)n));
       KNN_TRY(ar.alloc(&sidx, (size_t)n));
       KNN_TRY(ar.alloc(&cmin, (size_t)S.Rtot + 1));
       KNN_TRY(ar.alloc(&cmax, (size_t)S.Rtot + 1));
-      const bool idx_in_row = 4 * dp4 > d;
-      KNN_TRY(launch_cluster_layout(S.skeys, S.order, n, S.rows, dp4, idx_in_row, srows, sdist,
-                                    sidx, s));
+      const bool idx_in_row = !cols && 4 * dp4 > d;
+      KNN_TRY(launch_cluster_layout(S.skeys, S.order, n, S.rows, dp4, idx_in_row, cols, srows,
+                                    sdist, sidx, s));
       KNN_TRY(launch_cluster_minmax(S.off, sdist, S.Rtot, cmin, cmax, s));
       float4 *boxes = nullptr;
       if (narrow_rows(dp4)) {
@@ -560,6 +561,7 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       a.qorder = Q.order;
       a.qreps = Q.reps;
       a.boxes = boxes;
+      a.col_blocks = cols;
       a.slot_cl = slot_cl;
       a.qoff = Q.off;
       a.m = m;

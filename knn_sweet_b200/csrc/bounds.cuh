@@ -35,7 +35,8 @@ static __device__ __forceinline__ void bounds_filter_block(const float *dq, int 
                                     const float *__restrict__ scmax, float rq, int k, int d,
                                     int rs_pow2, int32_t id_base, uint64_t *skey,
                                     float *theta0_out, int32_t *rlist_out,
-                                    int32_t *rlen_out, float2 *chunk_out = nullptr) {
+                                    int32_t *rlen_out, float2 *chunk_out = nullptr,
+                                    float *lb_out = nullptr) {
   __shared__ int red_i[32];
   __shared__ unsigned red_u[32], red_l[32];
   __shared__ int kept_s;
@@ -159,8 +160,15 @@ static __device__ __forceinline__ void bounds_filter_block(const float *dq, int 
     }
   }
   const int kept = kept_s;
-  for (int j = tid; j < kept; j += nth)
-    rlist_out[j] = id_base + (int32_t)(skey[j] & 0xffffffffu);
+  for (int j = tid; j < kept; j += nth) {
+    const int c = (int32_t)(skey[j] & 0xffffffffu);
+    rlist_out[j] = id_base + c;
+    if (lb_out) {
+      // d(Rq, Rs) - radius, lowered by the rounding of both
+      const float dd = __uint_as_float((uint32_t)(skey[j] >> 32)), rr = scmax[c];
+      lb_out[j] = (dd - rr) - 2.0f * tol * (dd + rr);
+    }
+  }
   if (tid == 0) *rlen_out = kept;
   if (chunk_out && warp == 0) {
     // per chunk of 32 list entries: the first entry's d(Rq, Rs) (the list

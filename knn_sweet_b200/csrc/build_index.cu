@@ -410,6 +410,41 @@ __global__ void cluster_layout_kernel(const uint64_t *__restrict__ skeys,
   }
 }
 
+// The same in column blocks: one thread block per 32 positions; the rows are
+// read along their chunks and written along the positions, through shared
+// memory 32 chunks at a time (one column of padding: no bank conflicts).
+__global__ void __launch_bounds__(256)
+    cluster_layout_cols_kernel(const uint64_t *__restrict__ skeys,
+                               const int32_t *__restrict__ perm, int64_t n,
+                               const float4 *__restrict__ rows, int dp4,
+                               float4 *__restrict__ srows, float *__restrict__ sdist,
+                               int32_t *__restrict__ sidx) {
+  __shared__ float4 tile[32][33];
+  __shared__ int32_t src[32];
+  const int64_t base = (int64_t)blockIdx.x * 32;
+  const int cnt = (int)min((int64_t)32, n - base);
+  if (threadIdx.x < cnt) {
+    const int64_t p = base + threadIdx.x;
+    const int32_t r = perm[p];
+    src[threadIdx.x] = r;
+    sdist[p] = __uint_as_float((uint32_t)skeys[p]);
+    sidx[p] = r;
+  }
+  for (int c0 = 0; c0 < dp4; c0 += 32) {
+    const int nc = min(32, dp4 - c0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < cnt * nc; e += blockDim.x) {
+      const int r = e / nc, c = e - r * nc;
+      tile[c][r] = rows[(int64_t)src[r] * dp4 + c0 + c];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * nc; e += blockDim.x) {
+      const int c = e >> 5, r = e & 31;
+      if (r < cnt) srows[base * dp4 + (int64_t)(c0 + c) * kColStride + r] = tile[c][r];
+    }
+  }
+}
+
 // Offsets of every cluster in the sorted order (off[R] = n) from the sorted
 // keys, plus min / max member distance (the reference never fills the
 // reference-cluster radius: knnjoin.cu:391, defect B1).
@@ -687,7 +722,8 @@ __global__ void __launch_bounds__(512)
                          const float *__restrict__ scmax, int k, int d,
                          int rs_pow2, float *__restrict__ theta0,
                          int32_t *__restrict__ rlist,
-                         int32_t *__restrict__ rlen, float2 *__restrict__ clb) {
+                         int32_t *__restrict__ rlen, float2 *__restrict__ clb,
+                         float *__restrict__ rlb) {
   extern __shared__ uint64_t skey[];
   const int qc = blockIdx.x;
   if (qoff[qc + 1] == qoff[qc]) {  // empty query cluster
@@ -699,7 +735,8 @@ __global__ void __launch_bounds__(512)
   }
   bounds_filter_block(drr + (int64_t)qc * Rs, Rs, soff, sdist, scmax, qrad[qc], k, d, rs_pow2,
                       0, skey, theta0 + qc, rlist + (int64_t)qc * Rs, rlen + qc,
-                      clb ? clb + (int64_t)qc * ((Rs + 31) / 32) : nullptr);
+                      clb ? clb + (int64_t)qc * ((Rs + 31) / 32) : nullptr,
+                      rlb ? rlb + (int64_t)qc * Rs : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -944,12 +981,17 @@ int launch_cluster_sort(const int32_t *cl, const float *dr, int64_t n, int R,
 }
 
 int launch_cluster_layout(const uint64_t *skeys, const int32_t *perm, int64_t n,
-                          const float4 *rows, int dp4, bool idx_in_row,
+                          const float4 *rows, int dp4, bool idx_in_row, bool col_blocks,
                           float4 *srows, float *sdist, int32_t *sidx,
                           cudaStream_t s) {
   if (n == 0) return KNN_OK;
-  cluster_layout_kernel<<<grid_for(n * dp4, 256), 256, 0, s>>>(
-      skeys, perm, n, rows, dp4, idx_in_row, srows, sdist, sidx);
+  if (col_blocks) {
+    cluster_layout_cols_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(skeys, perm, n, rows, dp4,
+                                                                        srows, sdist, sidx);
+  } else {
+    cluster_layout_kernel<<<grid_for(n * dp4, 256), 256, 0, s>>>(
+        skeys, perm, n, rows, dp4, idx_in_row, srows, sdist, sidx);
+  }
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }
@@ -996,7 +1038,7 @@ int launch_bounds_filter(const float *drr, int Rq, int Rs, const float *qrad,
                          const int32_t *qoff, const int32_t *soff,
                          const float *sdist, const float *scmax, int k, int d,
                          float *theta0, int32_t *rlist, int32_t *rlen,
-                         float2 *clb, cudaStream_t s) {
+                         float2 *clb, float *rlb, cudaStream_t s) {
   int p2 = 1;
   while (p2 < Rs) p2 <<= 1;
   size_t smem = (size_t)p2 * sizeof(uint64_t);
@@ -1005,7 +1047,7 @@ int launch_bounds_filter(const float *drr, int Rq, int Rs, const float *qrad,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
   bounds_filter_kernel<<<Rq, 512, smem, s>>>(drr, Rq, Rs, qrad, qoff, soff, sdist,
-                                             scmax, k, d, p2, theta0, rlist, rlen, clb);
+                                             scmax, k, d, p2, theta0, rlist, rlen, clb, rlb);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }

@@ -32,6 +32,7 @@ struct ScanArgs {
   const float4 *sreps;      // Rs x dp4 reference representatives
   const float4 *srows;      // n x dp4, cluster-contiguous: ascending d(s,Rs),
                             // or (narrow rows) in block order
+  bool col_blocks;          // srows in column blocks (wide rows, col_block_at)
   const float4 *boxes;      // narrow rows: per block of 32 rows of a cluster the
                             // corners of its bounding box (block_slot; null:
                             // no block is skipped)
@@ -49,12 +50,15 @@ struct ScanArgs {
                             // list entries, x = d(Rq, Rs) of the chunk's first
                             // entry, y = the largest radius from that entry on
   int clb_stride;           // chunks per query cluster in clb
+  const float *rlb;         // optional (null: none): per list entry a lower bound
+                            // of d(Rq, Rs) - radius(Rs), as rlist
   const int64_t *rl_base;   // batched form: start of each query cluster's list
                             // in rlist (null: qc * Rs)
   const int64_t *qc_ref_base;  // batched form: subtracted from every output
                                // index of query cluster qc (null: 0)
   const int32_t *slot_list;    // optional: scan only these slots ...
   const unsigned *slot_count;  // ... *slot_count of them (device count);
+  int split_max;               // a block per query up to this many (launch_scan)
   int64_t slot_base;           // without a list: slots slot_base .. + m - 1
   int Rs;
   int64_t n_ref;            // reference points (0: unknown); with Rs it gives
@@ -111,7 +115,7 @@ int launch_chunk_slots(const int32_t *qorder, int64_t m, int first, int chunk_ro
                        uint32_t *keys, uint32_t *keys_out, int32_t *vals, int32_t *slots,
                        void *temp, size_t temp_bytes, cudaStream_t s);
 int launch_cluster_layout(const uint64_t *skeys, const int32_t *perm, int64_t n,
-                          const float4 *rows, int dp4, bool idx_in_row,
+                          const float4 *rows, int dp4, bool idx_in_row, bool col_blocks,
                           float4 *srows, float *sdist, int32_t *sidx,
                           cudaStream_t s);
 int launch_cluster_offsets(const uint64_t *skeys, int64_t n, int R, int32_t *off,
@@ -126,7 +130,19 @@ int launch_bounds_filter(const float *drr, int Rq, int Rs, const float *qrad,
                          const int32_t *qoff, const int32_t *soff,
                          const float *sdist, const float *scmax, int k, int d,
                          float *theta0, int32_t *rlist, int32_t *rlen,
-                         float2 *clb, cudaStream_t s);
+                         float2 *clb, float *rlb, cudaStream_t s);
+// Column blocks (rows of more than 8 floats): 32 consecutive rows of the
+// cluster-contiguous copy lie chunk by chunk, so that 32 lanes reading the
+// same 16-byte chunk of 32 members read 512 contiguous bytes.  First chunk of
+// position p, and the distance to its next chunk:
+__host__ __device__ inline int64_t col_block_at(int64_t p, int dp4) {
+  return (p & ~(int64_t)31) * dp4 + (p & 31);
+}
+constexpr int kColStride = 32;
+// float4 of the cluster-contiguous copy of n rows
+inline int64_t srows_count(int64_t n, int dp4, bool col_blocks) {
+  return (col_blocks ? (n + 31) / 32 * 32 : n) * dp4;
+}
 // Block order of narrow rows (at most 8 floats): within every cluster the
 // rows that lie near one another become neighbours in `out` (the sorted
 // position -> row map that perm holds by distance; out may be perm).
@@ -151,7 +167,8 @@ struct TileArgs {
   const int32_t *tiles;      // per tile: {query cluster, first slot, count,
                              // slot of the centre point}
   const int32_t *ntiles;     // device: number of tiles
-  const float4 *srows;       // n x dp4 reference rows, cluster-contiguous
+  const float4 *srows;       // n x dp4 reference rows, cluster-contiguous, in
+                             // column blocks
   const int32_t *sidx;       // n: original reference row
   const float4 *rrows;       // n x dp4 reference rows, original order
   const int32_t *soff;       // Rs + 1

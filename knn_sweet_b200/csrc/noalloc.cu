@@ -273,7 +273,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   p.share = self && p.Rq == p.Rs;
   p.trials = o.rep_trials;
   p.seed = o.seed;
-  p.idx_in_row = p.tmpl > 0 && 4 * p.dp4s > d;
+  p.idx_in_row = narrow_rows(p.tmpl) && 4 * p.dp4s > d;
   auto needs_pack = [&](const float *src) {
     return !(p.dp4s * 4 == d && (reinterpret_cast<uintptr_t>(src) & 15) == 0);
   };
@@ -319,7 +319,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
     rc = launch_block_order(Rp, p.dp4s, d, p.S.reps, p.S.skeys, p.S.off, p.S.perm, n, p.S.perm, s);
     if (rc != KNN_OK) return rc;
   }
-  rc = launch_cluster_layout(p.S.skeys, p.S.perm, n, Rp, p.dp4s, p.idx_in_row, p.srows,
+  rc = launch_cluster_layout(p.S.skeys, p.S.perm, n, Rp, p.dp4s, p.idx_in_row, false, p.srows,
                              p.sdist, p.sidx, s);
   if (rc == KNN_OK && boxes)
     rc = launch_block_boxes(p.srows, p.dp4s, d, p.S.skeys, p.S.off, n, boxes, s);
@@ -339,7 +339,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   if (rc == KNN_OK) rc = launch_rep_dist(Qb.reps, p.Rq, p.S.reps, p.Rs, p.dp4s, p.drr, s);
   if (rc == KNN_OK)
     rc = launch_bounds_filter(p.drr, p.Rq, p.Rs, p.qrad, Qb.off, p.S.off, p.sdist, p.cmax,
-                              k, d, p.theta0, p.rlist, p.rlen, nullptr, s);
+                              k, d, p.theta0, p.rlist, p.rlen, nullptr, nullptr, s);
   if (rc != KNN_OK) return rc;
   ScanArgs a{};
   a.qrows = Qp;

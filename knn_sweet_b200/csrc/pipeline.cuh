@@ -104,7 +104,7 @@ struct HostSink {
 struct RefSide {
   int64_t n = 0;
   int d = 0, dp4s = 0, tmpl = 0, Rs = 0;
-  bool idx_in_row = false;
+  bool idx_in_row = false, col_blocks = false;
   ClusterSet sset;
   const float4 *Rp = nullptr;  // packed rows, original order
   float4 *srows = nullptr;     // cluster-contiguous rows
@@ -128,6 +128,7 @@ struct QuerySide {
   const int *inexact = nullptr;
   float *qrad = nullptr, *drr = nullptr, *theta0 = nullptr;
   int32_t *slot_cl = nullptr, *rlist = nullptr, *rlen = nullptr;
+  float *rlb = nullptr;   // per list entry: d(Rq, Rs) less the radius of Rs
   float2 *clb = nullptr;  // per list chunk: first d(Rq, Rs), largest radius from it on
 };
 

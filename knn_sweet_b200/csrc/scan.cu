@@ -12,7 +12,12 @@
 //     member can be within theta (the reference's first-member `break`,
 //     knnjoin.cu:797); the survivors are visited nearest first (a warp sort
 //     on D), so the running k-th distance theta falls early.
-//   - Members are stored contiguously, ascending by d(s, Rs).  Members within
+//   - Rows of more than 8 floats: members are stored contiguously, ascending
+//     by d(s, Rs), in column blocks of 32 rows (the same chunk of 32 members
+//     is 512 contiguous bytes; a row per lane cost 32 cache lines per load and
+//     bound the scan: N = 10^6, d = 32, k = 32: 5.5 -> 3.1 ms with the list's
+//     lower bounds below; N = 400,000, d = 128, k = 100: 2.5 -> 1.4).
+//     Members within
 //     theta of q satisfy |D - d(s,Rs)| <= theta (knnjoin.cu:796-801), a
 //     contiguous band.  A warp-wide 32-ary search finds (to within 31
 //     members) where the band starts; the warp walks it 32 members per step
@@ -81,6 +86,7 @@ struct TopKBase {
   __device__ __forceinline__ unsigned *stat() const {
     return reinterpret_cast<unsigned *>(buf + kStatOff);
   }
+  static constexpr int kLostAt = kLostOff, kStatAt = kStatOff;
   __device__ __forceinline__ void count(int which, unsigned v, int lane) const {
     if (lane == 0) stat()[which] += v;
   }
@@ -180,6 +186,8 @@ struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3> {
     }
   }
 
+  // The candidates into buf[0..n) for another warp; returns n.
+  __device__ __forceinline__ int expose(int lane) { return sorted(lane, 0); }
   // The candidates, sorted, into buf[0..n); returns n.
   __device__ __forceinline__ int sorted(int lane, int) {
     __syncwarp();
@@ -322,6 +330,8 @@ struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
     set_band_threshold(__uint_as_float(T), d);
   }
 
+  // The candidates are in buf[0..nbuf) already.
+  __device__ __forceinline__ int expose(int) { return nbuf; }
   // End of the query: nothing to do before sorted().
   __device__ __forceinline__ void finish(int, int) {}
 
@@ -572,6 +582,26 @@ struct QueryRow {
   __device__ __forceinline__ float dist2(const float4 *__restrict__ r, int) const {
     return dist2_rows<DP4>(v, r);
   }
+  // A row whose chunks lie `stride` float4 apart; only the first nch chunks
+  // hold coordinates (the padding behind them would add exact zeros).
+  __device__ __forceinline__ float dist2_chunks(const float4 *__restrict__ r, int stride,
+                                                int nch) const {
+    float4 row[DP4];
+#pragma unroll
+    for (int c = 0; c < DP4; c++)
+      if (c < nch) row[c] = r[c * stride];
+    float acc = 0.0f;
+#pragma unroll
+    for (int c = 0; c < DP4; c++)
+      if (c < nch) {
+        float t;
+        t = __fsub_rn(v[c].x, row[c].x); acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(v[c].y, row[c].y); acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(v[c].z, row[c].z); acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(v[c].w, row[c].w); acc = __fmaf_rn(t, t, acc);
+      }
+    return acc;
+  }
   // Member row (already in registers): distance and (IDXROW) the index
   // stored in the row's last pad float.
   __device__ __forceinline__ float dist2_member(const float4 (&row)[DP4],
@@ -606,8 +636,19 @@ struct QueryRow<0, IDXROW> {
     __syncwarp();
     v = slot;
   }
-  __device__ __forceinline__ float dist2(const float4 *__restrict__ r, int dp4) const {
-    return dist2_rows_rt(v, r, dp4);
+  __device__ __forceinline__ float dist2_chunks(const float4 *__restrict__ r, int stride,
+                                                int nch) const {
+    float acc = 0.0f;
+#pragma unroll 4
+    for (int c = 0; c < nch; c++) {
+      const float4 u = v[c], s = r[(size_t)c * stride];
+      float t;
+      t = __fsub_rn(u.x, s.x); acc = __fmaf_rn(t, t, acc);
+      t = __fsub_rn(u.y, s.y); acc = __fmaf_rn(t, t, acc);
+      t = __fsub_rn(u.z, s.z); acc = __fmaf_rn(t, t, acc);
+      t = __fsub_rn(u.w, s.w); acc = __fmaf_rn(t, t, acc);
+    }
+    return acc;
   }
 };
 
@@ -620,32 +661,6 @@ struct QueryRow<0, IDXROW> {
 #ifndef KNN_TARGET_WARPS_WIDE
 #define KNN_TARGET_WARPS_WIDE 16
 #endif
-// Traversal choices (compile-time): visit a chunk's clusters nearest d(q,Rs)
-// first, and walk each band outward from d(s,Rs) ~ d(q,Rs).
-#ifndef KNN_ORDER_BY_D
-#define KNN_ORDER_BY_D 1
-#endif
-#ifndef KNN_WALK_OUTWARD
-#define KNN_WALK_OUTWARD 0
-#endif
-// Visits take a cluster's bounds and member range from the lanes that tested
-// it (loaded once per batch of 32 candidate clusters) and start the band
-// walk from the coarse member search (1); or reload them per visit and
-// search to the exact band edge (0).
-#ifndef KNN_VISIT_META
-#define KNN_VISIT_META 1
-#endif
-
-#ifndef KNN_INDEX32
-#define KNN_INDEX32 1
-#endif
-
-// The query's slot, row and cluster wait out the walk in shared memory (1)
-// or in registers (0).
-#ifndef KNN_SIDE_WORDS
-#define KNN_SIDE_WORDS 1
-#endif
-
 // Largest k kept in a register list (one key per lane): up to 24, so that
 // 8 of the 32 slots or more hold the FP32 band behind the k-th; larger k use
 // the shared-memory candidate set.
@@ -681,6 +696,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
   constexpr bool kWideRows = DP4 == 0 || DP4 >= 4;
   // narrow rows: members in block order, blocks of 32 skipped by their boxes
   constexpr bool kBlocks = DP4 == 1 || DP4 == 2;
+  const int nch = (a.d + 3) >> 2;  // chunks of a row that hold coordinates
   // statistics: per-lane 32-bit counts folded once per query into per-block
   // shared counters, added to the global ones at exit
   __shared__ unsigned long long blk_ctr[kScanCounters];
@@ -688,10 +704,28 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
   if (lane < kStatWords) tk.stat()[lane] = 0;
   __syncthreads();
 
+  // Few queries of wide rows (at most split_max): the block's warps share one
+  // query, each takes every WARPS-th cluster of its list, all tighten one
+  // threshold (s_thr, distance bits), and warp 0 merges their candidates
+  __shared__ unsigned s_thr;
+  __shared__ long long s_slot;
+  const bool split =
+      kWideRows &&
+      (a.slot_list ? (int64_t)*a.slot_count : a.m) <= (int64_t)a.split_max;
   for (;;) {
     long long slot = 0;
-    if (lane == 0) slot = (long long)atomicAdd(a.work_counter, 1ull);
-    slot = __shfl_sync(kFull, slot, 0);
+    if (split) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        s_slot = (long long)atomicAdd(a.work_counter, 1ull);
+        s_thr = 0x7f800000u;
+      }
+      __syncthreads();
+      slot = s_slot;
+    } else {
+      if (lane == 0) slot = (long long)atomicAdd(a.work_counter, 1ull);
+      slot = __shfl_sync(kFull, slot, 0);
+    }
     if (a.slot_list) {
       if (slot >= (long long)*a.slot_count) break;
       slot = a.slot_list[slot];
@@ -702,15 +736,12 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     }
     const int64_t q = a.qorder[slot];
     const int qc = a.slot_cl[slot];
-#if KNN_SIDE_WORDS
     if (lane == 0) {
       unsigned *sw = tk.stat();
       sw[kSideSlot] = (unsigned)slot;
       sw[kSideQuery] = (unsigned)q;
       sw[kSideCluster] = (unsigned)qc;
-      sw[kSideDq] = a.qkeys ? (uint32_t)a.qkeys[slot] : 0x7f800000u;  // +inf: no exit
     }
-#endif
     QueryRow<DP4, IDXROW> qr;
     qr.load(a.qrows, q, dp4, qslot);
     // the query's distance to its representative: slots of narrow rows are in
@@ -718,57 +749,47 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     float dq = __int_as_float(0x7f800000);
     if constexpr (kBlocks) dq = sqrtf(qr.dist2(a.qreps + (int64_t)qc * DP4, DP4));
     else if (a.qkeys) dq = __uint_as_float((uint32_t)a.qkeys[slot]);
+    if (lane == 0) tk.stat()[kSideDq] = __float_as_uint(dq);  // +inf: no early exit
     tk.reset(query_theta0(a, dq, qc, tol), lane);
+    __syncwarp();
 
-    // one band step: lane's member p of the cluster at `start`, kept when
-    // its distance to the representative lies in [lo_v, hi_v]
-    auto step = [&](int start, int p, bool valid, float lo_v, float hi_v) -> float {
-#if KNN_INDEX32
-      // row indices fit 32 bits (the result indices are int32): unsigned
-      // offsets make every address one wide multiply-add
+    // one step: lane's member p of the cluster at `start`, if `in`.  Row
+    // indices fit 32 bits (the result indices are int32): unsigned offsets make
+    // every address one wide multiply-add
+    auto step = [&](int start, int p, bool in) {
       const unsigned gp = (unsigned)(start + p);
-#else
-      const int64_t gp = (int64_t)start + p;
-#endif
-      float dsv = 0.0f, v = 0.0f;
+      float v = 0.0f;
       int32_t idx = 0;
-      bool inb;
-      if constexpr (kBlocks) {
-        inb = valid;
-        if (inb) {
-          float4 row[DP4];
-#pragma unroll
-          for (int c = 0; c < DP4; c++) row[c] = a.srows[(size_t)gp * DP4 + c];
-          v = qr.dist2_member(row, &idx);
-        }
-      } else if constexpr (DP4 > 0) {
-        dsv = valid ? a.sdist[gp] : 0.0f;
-        inb = valid && dsv >= lo_v && dsv <= hi_v;
-        if (inb) {
-          float4 row[DP4];
-#pragma unroll
-          for (int c = 0; c < DP4; c++) row[c] = a.srows[(size_t)gp * DP4 + c];
-          v = qr.dist2_member(row, &idx);
-        }
-      } else {
-        dsv = valid ? a.sdist[gp] : 0.0f;
-        inb = valid && dsv >= lo_v && dsv <= hi_v;
-        if (inb) v = qr.dist2(a.srows + (size_t)gp * dp4, dp4);
-      }
       bool pass = false;
-      if (inb) {
+      if (in) {
+        // the index is loaded with the row, not after its distance: one
+        // dependent round trip less per step
+        if constexpr (kBlocks) {
+          if constexpr (!IDXROW) idx = a.sidx[gp];
+          float4 row[DP4];
+#pragma unroll
+          for (int c = 0; c < DP4; c++) row[c] = a.srows[(size_t)gp * DP4 + c];
+          int32_t id = idx;
+          v = qr.dist2_member(row, &id);
+          if constexpr (IDXROW) idx = id;
+        } else {
+          idx = a.sidx[gp];
+          v = qr.dist2_chunks(
+              a.srows + (a.col_blocks ? col_block_at(gp, dp4) : (int64_t)gp * dp4),
+              a.col_blocks ? kColStride : 1, nch);
+        }
         evals++;
         pass = v <= tk.thr_d2;
-        if (!IDXROW && pass) idx = a.sidx[gp];
       }
       topk_offer(tk, pass, v, idx, lane, a.d);
-      return dsv;
     };
 
     const int nr = a.rlen[qc];
     const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
-    for (int base = 0; base < nr; base += 32) {
-#if KNN_CHUNK_EXIT && KNN_SIDE_WORDS
+    // (split: entry j of the list is warp j % WARPS's)
+    const int every = split ? WARPS : 1, first = split ? w : 0;
+    for (int base = 0; base < nr; base += 32 * every) {
+#if KNN_CHUNK_EXIT
       // the rest of the list is prunable when even its nearest cluster
       // (the list is ascending in d(Rq,Rs)) lies beyond theta for the
       // largest remaining radius: d(q,Rs) - cmax >= d(Rq,Rs) - d(q,Rq) -
@@ -781,25 +802,37 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const float2 cb = a.clb[(size_t)sw[kSideCluster] * a.clb_stride + (base >> 5)];
         const float dqv = __uint_as_float(sw[kSideDq]), th = tk.theta;
         if (cb.x - dqv - cb.y > th + 2.0f * tol * (cb.x + dqv + cb.y + th)) {
-          tk.count(kStatPruned, (unsigned)(nr - base), lane);
+          tk.count(kStatPruned, (unsigned)(max(nr - base - first, 0) + every - 1) / every, lane);
           break;
         }
       }
 #endif
-      const int j = base + lane;
+      const int j = base + lane * every + first;
+      const int batch = min(32, (max(nr - base - first, 0) + every - 1) / every);
+      // a cluster whose d(Rq,Rs) less its radius is beyond theta + d(q,Rq) is
+      // out without the distance to its representative (a gathered row per
+      // lane); most batches of a long list end here, at one coalesced load
+      bool listed = j < nr;
+      if (a.rlb) {
+        const float dqv = __uint_as_float(tk.stat()[kSideDq]), th = tk.theta;
+        if (listed)
+          listed = !(a.rlb[(size_t)(rl - a.rlist) + j] - dqv > th + 2.0f * tol * (dqv + th));
+        if (!__any_sync(kFull, listed)) {
+          tk.count(kStatPruned, (unsigned)batch, lane);
+          continue;
+        }
+      }
       int rs = 0;
       float D = 0.0f;
       bool alive = false;
-#if KNN_VISIT_META
       float cmx = 0.0f, cmn = 0.0f;
       int cst = 0, cnn = 0;
-#endif
-      if (j < nr) {
+      if (listed) {
         rs = rl[j];
-        D = sqrtf(qr.dist2(a.sreps + (int64_t)rs * dp4, dp4));
+        if constexpr (kBlocks) D = sqrtf(qr.dist2(a.sreps + (int64_t)rs * dp4, dp4));
+        else D = sqrtf(qr.dist2_chunks(a.sreps + (int64_t)rs * dp4, 1, nch));
         const float th = tk.theta;
         const float slack = tol * (2.0f * D + 2.0f * th);
-#if KNN_VISIT_META
         cmx = a.cmax[rs];
         cmn = a.cmin[rs];
         alive = !(D - cmx > th + slack) && !(D + th + slack < cmn);
@@ -807,14 +840,10 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           cst = a.soff[rs];
           cnn = a.soff[rs + 1] - cst;
         }
-#else
-        alive = !(D - a.cmax[rs] > th + slack) && !(D + th + slack < a.cmin[rs]);
-#endif
       }
-      // visit this chunk's surviving clusters: in list order (by rep-rep
-      // distance) or, with KNN_ORDER_BY_D, nearest d(q, Rs) first
+      // visit this chunk's surviving clusters, nearest d(q, Rs) first
       unsigned amask = __ballot_sync(kFull, alive);
-      tk.count(kStatPruned, (unsigned)(min(32, nr - base) - __popc(amask)), lane);
+      tk.count(kStatPruned, (unsigned)(batch - __popc(amask)), lane);
       if (amask == 0) continue;  // warp-uniform: nothing to visit in this batch
       const int nalive = __popc(amask);
       float dkey = alive ? D : __int_as_float(0x7f800000);
@@ -822,7 +851,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       // (bitonic network over the 32 lanes, ties to the lower lane: less work
       // per visited cluster); wider rows pick the nearest remaining cluster
       // by a warp arg-min per visit (measured faster there).
-      constexpr bool kSortBatch = KNN_ORDER_BY_D != 0 && DP4 >= 1 && DP4 <= 2;
+      constexpr bool kSortBatch = DP4 >= 1 && DP4 <= 2;
       float sv = dkey;
       int sl = lane;
       if (kSortBatch && nalive > 1) {  // a single survivor needs no order
@@ -847,7 +876,6 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           src = nalive > 1 ? __shfl_sync(kFull, sl, rank) : __ffs(amask) - 1;
         } else {
           src = __ffs(amask) - 1;
-#if KNN_ORDER_BY_D
           if (amask & (amask - 1)) {
             float mv = dkey;
             int ml = lane;
@@ -863,17 +891,21 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
             src = ml;
           }
           if (lane == src) dkey = __int_as_float(0x7f800000);
-#endif
           amask &= ~(1u << src);
         }
         const float Dc = __shfl_sync(kFull, D, src);
-#if KNN_VISIT_META
         const float cmax_c = __shfl_sync(kFull, cmx, src);
         const float cmin_c = __shfl_sync(kFull, cmn, src);
-#else
-        const int c = __shfl_sync(kFull, rs, src);
-        const float cmax_c = a.cmax[c], cmin_c = a.cmin[c];
-#endif
+        if (split) {
+          unsigned t = 0;
+          if (lane == 0) t = min(atomicMin(&s_thr, __float_as_uint(tk.thr_d2)),
+                                 __float_as_uint(tk.thr_d2));
+          const float tv = __uint_as_float(__shfl_sync(kFull, t, 0));
+          if (tv < tk.thr_d2) {
+            tk.thr_d2 = tv;
+            tk.theta = sqrtf(tv);
+          }
+        }
         float th = tk.theta;
         float slack = tol * (2.0f * Dc + 2.0f * th);
         if (Dc - cmax_c > th + slack || Dc + th + slack < cmin_c) {
@@ -881,13 +913,8 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           continue;
         }
         tk.count(kStatVisited, 1, lane);
-#if KNN_VISIT_META
         const int start = __shfl_sync(kFull, cst, src);
         const int n_c = __shfl_sync(kFull, cnn, src);
-#else
-        const int start = a.soff[c];
-        const int n_c = a.soff[c + 1] - start;
-#endif
         if constexpr (kBlocks) {
           // a lane per block of 32 members: the blocks whose box comes within
           // the threshold, in order, as long as they still do
@@ -912,76 +939,62 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
               todo &= todo - 1;
               if (__shfl_sync(kFull, bd, t) > tk.thr_d2) continue;
               const int p = 32 * (b0 + t) + lane;
-              step(start, p, p < n_c, 0.0f, 0.0f);
+              step(start, p, p < n_c);
             }
           }
           continue;
         }
-#if KNN_WALK_OUTWARD
-        // members below `mid` have d(s,Rs) < Dc, from `mid` on >= Dc; walk
-        // outward from there, alternately up and down
-        const int mid = warp_lower_bound(a.sdist + start, n_c, Dc, lane);
-        int up = mid, dn = mid;
-        bool go_up = up < n_c, go_dn = dn > 0;
-        while (go_up || go_dn) {
-          if (go_up) {
-            th = tk.theta;
-            slack = tol * (2.0f * Dc + 2.0f * th);
-            const float hi_v = Dc + th + slack;
-            const int p = up + lane;
-            const bool valid = p < n_c;
-            const float dsv = step(start, p, valid, -1.0f, hi_v);
-            const bool past = !valid || dsv > hi_v;
-            up += 32;
-            if (__shfl_sync(kFull, past, 31) || up >= n_c) go_up = false;
-          }
-          if (go_dn) {
-            th = tk.theta;
-            slack = tol * (2.0f * Dc + 2.0f * th);
-            const float lo_v = Dc - th - slack;
-            const int p = dn - 32 + lane;
-            const bool valid = p >= 0;
-            const float dsv = step(start, p, valid, lo_v, __int_as_float(0x7f800000));
-            const bool past = !valid || dsv < lo_v;
-            dn -= 32;
-            if (__shfl_sync(kFull, past, 0) || dn <= 0) go_dn = false;
-          }
-        }
-#else
         // one direction: from the lower band edge up (no search when the band
         // starts below the cluster's nearest member)
         const float lo_edge = Dc - th - slack;
-#if KNN_VISIT_META
         const int lo = lo_edge <= cmin_c ? 0 : warp_lower_bound_coarse(a.sdist + start, n_c, lo_edge, lane);
-#else
-        const int lo = lo_edge <= cmin_c ? 0 : warp_lower_bound(a.sdist + start, n_c, lo_edge, lane);
-#endif
+        const float inf = __int_as_float(0x7f800000);
+        float dsv = lo + lane < n_c ? a.sdist[start + lo + lane] : inf;
         for (int p0 = lo; p0 < n_c; p0 += 32) {
           th = tk.theta;
           slack = tol * (2.0f * Dc + 2.0f * th);
           const float hi_v = Dc + th + slack, lo_v = Dc - th - slack;
           const int p = p0 + lane;
-          const bool valid = p < n_c;
-          const float dsv = step(start, p, valid, lo_v, hi_v);
-          const bool past = !valid || dsv > hi_v;
-          if (__shfl_sync(kFull, past, 31)) break;
+          const float ds = dsv;
+          // the next step's band distances come while this one's rows do
+          dsv = p + 32 < n_c ? a.sdist[start + p + 32] : inf;
+          step(start, p, p < n_c && ds >= lo_v && ds <= hi_v);
+          if (__shfl_sync(kFull, ds > hi_v, 31)) break;
         }
-#endif
       }
     }
     tk.finish(lane, a.d);
-#if KNN_SIDE_WORDS
+    if (split) {
+      // the other warps' candidates, into warp 0's
+      if (w > 0) {
+        const int cnt = tk.expose(lane);
+        if (lane == 0) tk.stat()[kSideQuery] = (unsigned)cnt;
+      }
+      __syncthreads();
+      if (w == 0) {
+        for (int o = 1; o < WARPS; o++) {
+          const uint64_t *ob = keys_base + (size_t)o * TK::kSmemKeys;
+          const int cnt = (int)reinterpret_cast<const unsigned *>(ob + TK::kStatAt)[kSideQuery];
+          const float ol = *reinterpret_cast<const float *>(ob + TK::kLostAt);
+          __syncwarp();
+          if (lane == 0) *tk.lostmin() = fminf(*tk.lostmin(), ol);
+          for (int e = 0; e < cnt; e += 32) {
+            const uint64_t key = e + lane < cnt ? ob[e + lane] : kKeyMax;
+            const float v = key_d2(key);
+            topk_offer(tk, e + lane < cnt && v <= tk.thr_d2, v, key_idx(key), lane, a.d);
+          }
+        }
+        tk.finish(lane, a.d);
+      }
+    }
     __syncwarp();
-    {
+    if (!split || w == 0) {
       const unsigned *sw = tk.stat();
       const int32_t e_slot = (int32_t)sw[kSideSlot];
       const int64_t e_q = (int64_t)sw[kSideQuery];
       const int e_qc = (int)sw[kSideCluster];
       tk.count(kStatChecked, emit_query(tk, a, e_slot, e_q, e_qc, lane), lane);
     }
-#else
-    tk.count(kStatChecked, emit_query(tk, a, (int32_t)slot, q, qc, lane), lane);
-#endif
     __syncwarp();
     if (a.counters) {
 #pragma unroll
@@ -997,13 +1010,22 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       }
     }
     __syncwarp();
-    if (lane < kStatWords) tk.stat()[lane] = 0;
+    if (lane < kSideSlot) tk.stat()[lane] = 0;  // (warp 0 may still read the side words)
     evals = 0;
   }
   __syncthreads();
   if (a.counters && threadIdx.x < kScanCounters)
     atomicAdd(a.counters + threadIdx.x, blk_ctr[threadIdx.x]);
 }
+
+// Queries of wide rows up to this many times the resident blocks get a block
+// each (scan_kernel's split): a warp per query then leaves the chip waiting
+// for the query with the most clusters to visit.  200,003 reference rows,
+// d = 17, k = 10, 1,013 queries: search 971 -> 289 us; 100 queries 746 -> 141;
+// 100,000 rows, d = 64, 2,000 queries (8 times): 2430 -> 1526.  With short
+// lists the blocks' own start and merge weigh more (2,000 queries over 72
+// clusters: 43 -> 104), hence 4 there.
+static int split_waves(int Rs) { return Rs >= 256 ? 8 : 4; }
 
 template <int DP4, bool IDXROW, int L, int WARPS>
 static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
@@ -1017,11 +1039,13 @@ static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
   int per_sm = 0;
   KNN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
   if (per_sm < 1) per_sm = 1;
-  const int64_t want = (a.m + WARPS - 1) / WARPS;
   int64_t grid = (int64_t)num_sms * per_sm;
+  ScanArgs b = a;
+  b.split_max = (int)(split_waves(a.Rs) * grid);
+  const int64_t want = a.m <= b.split_max ? a.m : (a.m + WARPS - 1) / WARPS;
   if (grid > want) grid = want;
   if (grid < 1) grid = 1;
-  kern<<<(int)grid, WARPS * 32, smem, s>>>(a);
+  kern<<<(int)grid, WARPS * 32, smem, s>>>(b);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }
@@ -1666,10 +1690,10 @@ __device__ void band_cut(BandEntry *e, int *cnt, BandEntry *thr, int need) {
 // the scan kernels' value for the same pair (their padded coordinates add
 // exact zeros).
 __device__ __forceinline__ float band_dist2(const float *__restrict__ q,
-                                            const float *__restrict__ r, int d) {
+                                            const float *__restrict__ r, int d, int stride = 1) {
   float acc = 0.0f;
   for (int c = 0; c < d; c++) {
-    const float t = __fsub_rn(q[c], r[c]);
+    const float t = __fsub_rn(q[c], r[(size_t)(c >> 2) * (4 * stride) + (c & 3)]);
     acc = __fmaf_rn(t, t, acc);
   }
   return acc;
@@ -1716,7 +1740,11 @@ __global__ void __launch_bounds__(kBandThreads) band_resolve_kernel(const ScanAr
       // the same for all (the count itself may move on while others read it)
       int full = 0;
       if (in) {
-        const float v = band_dist2(qv, reinterpret_cast<const float *>(a.srows + gp * dp4), d);
+        const float v =
+            a.col_blocks
+                ? band_dist2(qv, reinterpret_cast<const float *>(a.srows + col_block_at(gp, dp4)),
+                             d, kColStride)
+                : band_dist2(qv, reinterpret_cast<const float *>(a.srows + gp * dp4), d);
         if (v >= lo && v <= hi) {
           const int32_t id = a.sidx[gp];
           const double w =
@@ -1862,10 +1890,8 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
                                 : launch_scan_l<1, false>(a, num_sms, s);
     case 2: return a.idx_in_row ? launch_scan_l<2, true>(a, num_sms, s)
                                 : launch_scan_l<2, false>(a, num_sms, s);
-    case 4: return a.idx_in_row ? launch_scan_l<4, true>(a, num_sms, s)
-                                : launch_scan_l<4, false>(a, num_sms, s);
-    case 8: return a.idx_in_row ? launch_scan_l<8, true>(a, num_sms, s)
-                                : launch_scan_l<8, false>(a, num_sms, s);
+    case 4: return launch_scan_l<4, false>(a, num_sms, s);
+    case 8: return launch_scan_l<8, false>(a, num_sms, s);
     default: return launch_scan_l<0, false>(a, num_sms, s);
   }
 }

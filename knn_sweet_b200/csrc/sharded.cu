@@ -105,13 +105,14 @@ int replicate_sides(Arena &ar, int g, int g0, const RefSide &R, const QuerySide 
   R2->tmpl = R.tmpl;
   R2->Rs = Rs;
   R2->idx_in_row = R.idx_in_row;
+  R2->col_blocks = R.col_blocks;
   R2->sset.R = Rs;
   float4 *rp;
   KNN_TRY(replicate(ar, g, g0, R.Rp, (size_t)n * dp4, s, &rp));
   R2->Rp = rp;
   KNN_TRY(replicate(ar, g, g0, R.sset.reps, (size_t)Rs * dp4, s, &R2->sset.reps));
   KNN_TRY(replicate(ar, g, g0, R.sset.off, (size_t)Rs + 1, s, &R2->sset.off));
-  KNN_TRY(replicate(ar, g, g0, R.srows, (size_t)n * dp4, s, &R2->srows));
+  KNN_TRY(replicate(ar, g, g0, R.srows, (size_t)srows_count(n, dp4, R.col_blocks), s, &R2->srows));
   KNN_TRY(replicate(ar, g, g0, R.sdist, (size_t)n, s, &R2->sdist));
   KNN_TRY(replicate(ar, g, g0, R.sidx, (size_t)n, s, &R2->sidx));
   KNN_TRY(replicate(ar, g, g0, R.boxes, (size_t)block_count(n, Rs) * 2 * dp4, s, &R2->boxes));
@@ -148,6 +149,7 @@ int replicate_sides(Arena &ar, int g, int g0, const RefSide &R, const QuerySide 
   KNN_TRY(replicate(ar, g, g0, Q.qset.skeys, (size_t)m, s, &Q2->qset.skeys));
   KNN_TRY(replicate(ar, g, g0, Q.rlist, (size_t)Rq * Rs, s, &Q2->rlist));
   KNN_TRY(replicate(ar, g, g0, Q.rlen, (size_t)Rq, s, &Q2->rlen));
+  KNN_TRY(replicate(ar, g, g0, Q.rlb, (size_t)Rq * Rs, s, &Q2->rlb));
   if (Q.clb)
     KNN_TRY(replicate(ar, g, g0, Q.clb, (size_t)Rq * ((Rs + 31) / 32), s, &Q2->clb));
   return KNN_OK;

@@ -51,6 +51,13 @@ namespace {
 #endif
 // (first batch 2 / 4 / 8: C3 search 10.5 / 11.1 / 11.2 ms, C2 11.9 / 4.2 /
 // 4.6 ms; growth 3 / 4 / 6: C2 4.29 / 4.24 / 4.13-4.16 ms, C3 unchanged)
+// Members that a tile may stream in one batch of clusters (N = 10^6, d = 32,
+// k = 32, search of five data sets in ms, no limit 3.7 / 8.0 / 9.8 / 3.4 / 4.3;
+// 32,768: 3.9 / 4.5 / 5.5 / 3.6 / 4.5; 16,384: 3.8 / 4.2 / 5.6 / 3.5 / 4.3;
+// 8,192: 3.8 / 4.3 / 5.5 / 3.5 / 4.6; 4,096 hands a third of all queries back).
+#ifndef KNN_TILE_MAX_RUN
+#define KNN_TILE_MAX_RUN 16384
+#endif
 #ifndef KNN_TILE_GROW
 #define KNN_TILE_GROW 6
 #endif
@@ -192,6 +199,63 @@ __device__ __forceinline__ void stage_tile(unsigned char *tile, const float *sc,
   }
 }
 
+// The same for member rows in column blocks: thread t takes row t % kTM and
+// (with NT = 2 kTM) every other 16-byte group of its columns, so that a warp
+// reads 512 contiguous bytes per chunk, stores 16-byte groups of consecutive
+// rows without bank conflicts and adds up its row's sums without shuffles.
+// pos: the row's position (negative: zeros).  The second half's sums go to
+// part[0..3 kTM) and are added by the caller's barrier (finish_sums).
+template <int NT>
+__device__ __forceinline__ void stage_members(unsigned char *tile, const float *sc, int KD, int d,
+                                              int dp4, const float4 *__restrict__ srows,
+                                              int64_t pos, float *o_n, float *o_e, float *o_t,
+                                              float *part) {
+  constexpr int H = NT / kTM;
+  const int r = threadIdx.x & (kTM - 1), h = threadIdx.x / kTM;
+  const float4 *row = srows + (pos >= 0 ? col_block_at(pos, dp4) : 0);
+  float sn = 0.0f, se = 0.0f, st = 0.0f;
+  const int G = KD >> 3;
+  for (int g0 = h; g0 < G; g0 += 4 * H) {
+    float4 c0[4], c1[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int ch = 2 * (g0 + u * H);
+      c0[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      c1[u] = c0[u];
+      if (pos >= 0) {
+        if (ch < dp4) c0[u] = row[(size_t)ch * kColStride];
+        if (ch + 1 < dp4) c1[u] = row[(size_t)(ch + 1) * kColStride];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int g = g0 + u * H, k0 = g << 3;
+      if (g >= G) break;
+      const float v[8] = {c0[u].x, c0[u].y, c0[u].z, c0[u].w,
+                          c1[u].x, c1[u].y, c1[u].z, c1[u].w};
+      __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const int kk = k0 + e;
+        const float x = (pos >= 0 && kk < d) ? __fsub_rn(v[e], sc[kk]) : 0.0f;
+        b[e] = __float2bfloat16_rn(x);
+        const float xr = __bfloat162float(b[e]);
+        const float df = __fsub_rn(x, xr);
+        sn = __fmaf_rn(x, x, sn);
+        se = __fmaf_rn(df, df, se);
+        st = __fmaf_rn(xr, xr, st);
+      }
+      *reinterpret_cast<uint4 *>(tile + tc::tile_offset(r, k0, KD)) =
+          *reinterpret_cast<const uint4 *>(b);
+    }
+  }
+  float *on = h == 0 ? o_n : part, *oe = h == 0 ? o_e : part + kTM,
+        *ot = h == 0 ? o_t : part + 2 * kTM;
+  on[r] = sn;
+  oe[r] = se;
+  ot[r] = st;
+}
+
 // Keeps the entries of a bound buffer (lu, pos: n entries in shared memory)
 // whose lower bound is at most the k-th smallest upper bound, or an upper
 // bound of it -- no entry beyond it can be among the k nearest; in place, by
@@ -316,6 +380,9 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
   uint64_t *mbar = reinterpret_cast<uint64_t *>(hist + 4 * 256);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 1);
   int32_t *s_tile = reinterpret_cast<int32_t *>(tmem_slot + 1);  // 4 ints
+  // second partial sums of the staged rows, in the histograms: those serve
+  // the compactions, which no staging overlaps
+  float *s_part = reinterpret_cast<float *>(hist);
   // warps 0-3: one query's buffer each (cap bound pairs, cap positions), a
   // query row and a histogram, for the compactions between member chunks
   // and the final re-ranking; warps 4-7 join the re-ranking only, once the
@@ -608,26 +675,34 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
         }
       }
 #endif
+      // a tile whose queries reach too far for this form (a cluster that spans
+      // distant groups of points: loose bounds, every member a candidate) goes
+      // to the FP32 scan as a whole, before it streams them: one such tile took
+      // as long as all others together
+      if (total > KNN_TILE_MAX_RUN) {
+        ovf = true;
+        break;
+      }
       // the runs, concatenated, in chunks of kTN rows
       for (int o = 0; o < total; o += kTN) {
         const int nr = min(kTN, total - o);
         const bool last_of_first = jb == 0 && o + kTN >= total;
-        stage_tile<NT>(
-            sb, sc, KD, d, dp4,
-            [&](int r) -> const float4 * {
-              if (r >= nr) return nullptr;
-              const int g = o + r;
-              int l = 0, h = kTN - 1;  // last run starting at or before g
-              while (l < h) {
-                const int md = (l + h + 1) >> 1;
-                if (s_roff[md] <= g) l = md;
-                else h = md - 1;
-              }
-              const int p = s_rlo[l] + (g - s_roff[l]);
-              s_pos[r] = p;
-              return a.srows + (size_t)p * dp4;
-            },
-            s_n, s_e, s_t);
+        {
+          const int r = tid & (kTM - 1);
+          int64_t p = -1;
+          if (r < nr) {
+            const int g = o + r;
+            int l = 0, h = kTN - 1;  // last run starting at or before g
+            while (l < h) {
+              const int md = (l + h + 1) >> 1;
+              if (s_roff[md] <= g) l = md;
+              else h = md - 1;
+            }
+            p = s_rlo[l] + (g - s_roff[l]);
+            if (tid < kTM) s_pos[r] = (int32_t)p;
+          }
+          stage_members<NT>(sb, sc, KD, d, dp4, a.srows, p, s_n, s_e, s_t, s_part);
+        }
         tc::fence_proxy_async_smem();
         tc::fence_before_sync();
         __syncthreads();
@@ -642,6 +717,11 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
           tc::mma_commit(mbar);
         }
         // column scalars: |b|^2 (+inf on padding), |b - b~|, |b~|, position
+        if (NT > kTM && row_thread) {
+          s_n[tid] += s_part[tid];
+          s_e[tid] += s_part[kTM + tid];
+          s_t[tid] += s_part[2 * kTM + tid];
+        }
         if (row_thread)
           s_col[tid] = tid < nr ? make_float4(s_n[tid], sqrtf(s_e[tid]), sqrtf(s_t[tid]),
                                               __int_as_float(s_pos[tid]))
@@ -680,9 +760,15 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
         compact_rows(last_of_first ? k - 1 : lim);
         TILE_PROF(4);
         tc::fence_before_sync();
-        __syncthreads();  // the member tile, TMEM and column scalars are reused
+        // the member tile, TMEM and column scalars are reused; a tile without
+        // a query left that keeps its pairs is done
+        const bool none = __syncthreads_and(!valid || ovf) != 0;
         tc::fence_after_sync();
         TILE_PROF(5);
+        if (none) {
+          nb = nl - jb;
+          break;
+        }
       }
     }
     if (!ok) break;
@@ -724,8 +810,9 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
       if (!fb) {
         for (int e = lane; e < m1; e += 32) {
           const int p = w_pos[e];
-          const float d2 = dist2_cols(wq, a.srows + (size_t)p * dp4, d);
-          keys[e] = make_key(d2, a.sidx[p]);
+          const int32_t id = a.sidx[p];  // the row itself in its original place
+          const float d2 = dist2_cols(wq, a.rrows + (size_t)id * dp4, d);
+          keys[e] = make_key(d2, id);
         }
         if (lane == 0) refined += (unsigned long long)m1;
         __syncwarp();

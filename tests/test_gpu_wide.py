@@ -1,0 +1,68 @@
+"""Joins of wide rows (d > 8): members in column blocks of 32, the list's lower
+bounds, and the scan that gives a query a whole block when there are few.
+
+Sizes sit at the edges: one row more or less than a block, rows with one float
+in their last chunk, every top-k variant, few queries (a block each) and many
+(a warp each).
+"""
+import numpy as np
+import pytest
+
+from knn_sweet_b200 import knnjoin
+from tests.parity import assert_matches
+
+pytestmark = pytest.mark.gpu
+
+
+def _mix(rng, n, d, centres):
+    return (centres[rng.integers(0, len(centres), n)] +
+            0.5 * rng.standard_normal((n, d))).astype(np.float32)
+
+
+@pytest.mark.parametrize("d,k", [(9, 10), (16, 1), (17, 24), (17, 25), (31, 64), (33, 128),
+                                 (64, 200), (100, 300), (130, 600), (257, 5)])
+@pytest.mark.parametrize("m", [40, 3000])
+def test_wide_rows(cuda_device, oracle, d, k, m):
+    rng = np.random.default_rng(d * 1000 + k)
+    centres = rng.uniform(-3, 3, (12, d))
+    r, q = _mix(rng, 2001, d, centres), _mix(rng, m, d, centres)
+    idx, dist = knnjoin(q, r, k, sreps=90)
+    rows = rng.permutation(m)[:400]
+    oi, od = oracle.bruteforce_f64(q[rows], r, k)
+    assert_matches(idx[rows], dist[rows], oi, od)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 65])
+@pytest.mark.parametrize("precision", ["fp32", "bf16_refine"])
+def test_column_block_edges(cuda_device, oracle, n, precision):
+    rng = np.random.default_rng(n)
+    r = rng.standard_normal((n, 36)).astype(np.float32)
+    q = rng.standard_normal((200, 36)).astype(np.float32)
+    idx, dist = knnjoin(q, r, 7, sreps=min(n, 3), precision=precision)
+    oi, od = oracle.bruteforce_f64(q, r, 7)
+    assert_matches(idx, dist, oi, od)
+
+
+def test_few_queries_ties(cuda_device, oracle):
+    # a block per query: equal distances in several warps' shares
+    rng = np.random.default_rng(3)
+    r = rng.integers(0, 2, (4000, 12)).astype(np.float32)
+    q = rng.integers(0, 2, (33, 12)).astype(np.float32)
+    for k in (3, 20, 100):
+        idx, dist = knnjoin(q, r, k, sreps=64)
+        oi, od = oracle.bruteforce_f64(q, r, k)
+        assert_matches(idx, dist, oi, od, exact=True)
+
+
+def test_tile_that_reaches_too_far(cuda_device, oracle):
+    # one query cluster over two distant groups and every member a candidate:
+    # the tile goes back to the FP32 scan, with the same result
+    rng = np.random.default_rng(9)
+    r = np.concatenate([rng.standard_normal((20_000, 16)),
+                        rng.standard_normal((20_000, 16)) + 40.0]).astype(np.float32)
+    q = np.concatenate([rng.standard_normal((64, 16)),
+                        rng.standard_normal((64, 16)) + 40.0]).astype(np.float32)
+    idx, dist, st = knnjoin(q, r, 20, qreps=1, sreps=40, precision="bf16_refine", stats=True)
+    oi, od = oracle.bruteforce_f64(q, r, 20)
+    assert_matches(idx, dist, oi, od)
+    assert st.refine_fallbacks > 0
