@@ -381,6 +381,24 @@ int query_impl(const RefSide &R, bool share, const float *q, int64_t m, int32_t 
                cudaStream_t s, HostSink *sink, Arena &ar, EventSet &evs,
                unsigned long long *ctr);
 
+// The end of a call: the last event and, with `st`, the statistics.
+int finish_stats(int Rq, int Rs, HostSink *sink, unsigned long long *ctr, cudaStream_t s,
+                 EventSet &evs, knn_stats *st) {
+  KNN_TRY(evs.record(2, s));
+  if (st) {
+    KNN_TRY(read_stats(ctr, s, st));
+    if (sink && sink->done) KNN_CUDA_TRY(cudaStreamSynchronize(sink->copy));
+    st->pairs_pruned = st->pairs_total - st->dist_evals;
+    st->qreps_used = Rq;
+    st->sreps_used = Rs;
+    st->kernels_launched = launch_counter();
+    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_build, evs.ev[0], evs.ev[1]));
+    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_search, evs.ev[1], evs.ev[2]));
+    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_total, evs.ev[0], evs.ev[2]));
+  }
+  return KNN_OK;
+}
+
 int join_device_impl(const float *q, int64_t m, const float *r, int64_t n,
                      int32_t d, int32_t k, int32_t *out_idx, float *out_dist,
                      const knn_options *opt, knn_stats *st, cudaStream_t s,
@@ -414,6 +432,11 @@ int join_device_impl(const float *q, int64_t m, const float *r, int64_t n,
   unsigned long long *ctr;
   KNN_TRY(ar.alloc(&ctr, kCtrCount));
   KNN_CUDA_TRY(cudaMemsetAsync(ctr, 0, kCtrCount * sizeof(unsigned long long), s));
+  if (small_join_fits(m, n, d, o)) {
+    KNN_TRY(small_join(q, m, r, n, d, k, out_idx, out_dist, o, ar, ctr, s,
+                       st ? evs.ev[1] : nullptr));
+    return finish_stats(1, 1, sink, ctr, s, evs, st);
+  }
   RefSide R;
   KNN_TRY(build_ref_side(ar, ar, r, n, d, Rs, o, false, reinterpret_cast<int *>(ctr + kCtrErr),
                          s, &R));
@@ -732,19 +755,7 @@ int query_impl(const RefSide &R, bool share, const float *q, int64_t m, int32_t 
   KNN_TRY(build_query_side(R, share, q, m, k, o, ar, ctr, s, &Q));
   KNN_TRY(evs.record(1, s));
   KNN_TRY(search_clusters(R, Q, m, k, 0, Q.Rq, 0, m, out_idx, out_dist, o, s, sink, ar, ctr));
-  KNN_TRY(evs.record(2, s));
-  if (st) {
-    KNN_TRY(read_stats(ctr, s, st));
-    if (sink && sink->done) KNN_CUDA_TRY(cudaStreamSynchronize(sink->copy));
-    st->pairs_pruned = st->pairs_total - st->dist_evals;
-    st->qreps_used = Q.Rq;
-    st->sreps_used = R.Rs;
-    st->kernels_launched = launch_counter();
-    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_build, evs.ev[0], evs.ev[1]));
-    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_search, evs.ev[1], evs.ev[2]));
-    KNN_CUDA_TRY(cudaEventElapsedTime(&st->ms_total, evs.ev[0], evs.ev[2]));
-  }
-  return KNN_OK;
+  return finish_stats(Q.Rq, R.Rs, sink, ctr, s, evs, st);
 }
 
 // Index build / query (the reusable reference side).

@@ -501,74 +501,70 @@ __global__ void slot_cluster_kernel(const uint64_t *__restrict__ skeys,
 // bounding box.  Here every run of 1,024 positions is reordered, cluster by
 // cluster, along a Morton curve over the cluster's own extent (the ball of its
 // radius around its representative); a cluster that crosses a run's end is
-// ordered in parts.  One block per run, keys in shared memory: cluster (less
-// the run's first), Morton code, position.
+// ordered in parts.  One block per run, 32-bit keys: where the cluster starts
+// in the run, 12 bits of Morton code, the position (34 M points: 1.38 ms with
+// 64-bit keys sorted in shared memory, 0.81 with block_sort_u32).
 // ---------------------------------------------------------------------------
 constexpr int kOrderRun = 1024;
+constexpr int kOrderThreads = 256;
 
 template <int DP4>
-__global__ void __launch_bounds__(kOrderRun / 2)
+__global__ void __launch_bounds__(kOrderThreads)
     block_order_kernel(const float4 *__restrict__ rows, int d, const float4 *__restrict__ reps,
                        const uint64_t *__restrict__ skeys, const int32_t *__restrict__ off,
                        const int32_t *perm, int64_t n, int32_t *out) {
-  __shared__ uint64_t key[kOrderRun];
+  constexpr int E = kOrderRun / kOrderThreads;
+  __shared__ uint32_t sm[kOrderRun];
   __shared__ int32_t src[kOrderRun];
   const int64_t base = (int64_t)blockIdx.x * kOrderRun;
   const int cnt = (int)min((int64_t)kOrderRun, n - base);
-  const int c_first = (int)(skeys[base] >> 32);
-  const int bits = min(10, 30 / d);  // per coordinate
+  const int bits = 12 / d > 0 ? 12 / d : 1;  // per coordinate, of the first 12
   const float top = (float)((1 << bits) - 1);
-  for (int t = threadIdx.x; t < kOrderRun; t += blockDim.x) {
-    uint64_t k = kKeyMax;
+  // keys computed along the positions, sorted in blocked order (any
+  // assignment of keys to threads is as good before the sort)
+  uint32_t x[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int t = e * kOrderThreads + threadIdx.x;
+    x[e] = 0xffffffffu;
     if (t < cnt) {
       const int c = (int)(skeys[base + t] >> 32);
       const int32_t row = perm[base + t];
+      const int c0 = off[c];
       const float rad = __uint_as_float((uint32_t)skeys[off[c + 1] - 1]);
-      const float scale = rad > 0.0f ? 0.5f * top / rad : 0.0f;
-      float x[4 * DP4];
+      const float scale = rad > 0.0f ? 0.5f * (top + 1.0f) / rad : 0.0f;
+      float v[4 * DP4];
 #pragma unroll
-      for (int e = 0; e < DP4; e++) {
-        const float4 v = rows[(int64_t)row * DP4 + e], r = reps[(int64_t)c * DP4 + e];
-        x[4 * e] = v.x - r.x;
-        x[4 * e + 1] = v.y - r.y;
-        x[4 * e + 2] = v.z - r.z;
-        x[4 * e + 3] = v.w - r.w;
+      for (int h = 0; h < DP4; h++) {
+        const float4 a = rows[(int64_t)row * DP4 + h], r = reps[(int64_t)c * DP4 + h];
+        v[4 * h] = a.x - r.x;
+        v[4 * h + 1] = a.y - r.y;
+        v[4 * h + 2] = a.z - r.z;
+        v[4 * h + 3] = a.w - r.w;
       }
       uint32_t code = 0;
 #pragma unroll
-      for (int e = 0; e < 4 * DP4; e++)
-        if (e < d) {
+      for (int h = 0; h < 4 * DP4; h++)
+        if (h < d) {
           // (a NaN becomes 0: such a row may go anywhere)
-          const int q = (int)fminf(fmaxf(x[e] * scale + 0.5f * top, 0.0f), top);
-          for (int b = 0; b < bits; b++) code |= (uint32_t)((q >> b) & 1) << (b * d + e);
+          const int q =
+              (int)fminf(fmaxf(v[h] * scale + 0.5f * (top + 1.0f), 0.0f), top);
+          for (int b = 0; b < bits; b++) code |= (uint32_t)((q >> b) & 1) << (b * d + h);
         }
-      k = ((uint64_t)(uint32_t)(c - c_first) << 40) | ((uint64_t)code << 10) | (uint32_t)t;
+      const uint32_t start = (uint32_t)max((int64_t)c0 - base, (int64_t)0);
+      x[e] = (start << 22) | (code << 10) | (uint32_t)t;
       src[t] = row;
     }
-    key[t] = k;
   }
-  int p2 = 32;
-  while (p2 < cnt) p2 <<= 1;
+  block_sort_u32<E>(x, sm);
   __syncthreads();
-  for (int size = 2; size <= p2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const int t = threadIdx.x;
-      if (t < p2 / 2) {
-        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
-        const bool up = (i & size) == 0;
-        const uint64_t a = key[i], b = key[j];
-        if ((a > b) == up) {
-          key[i] = b;
-          key[j] = a;
-        }
-      }
-      // strides below a warp's 64 keys stay inside the warp
-      if (stride > 32) __syncthreads();
-      else __syncwarp();
-    }
-    __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int i = E * threadIdx.x + e;
+    if (i < cnt) sm[i] = (uint32_t)src[x[e] & 1023u];
   }
-  for (int t = threadIdx.x; t < cnt; t += blockDim.x) out[base + t] = src[(int)(key[t] & 1023u)];
+  __syncthreads();
+  for (int i = threadIdx.x; i < cnt; i += kOrderThreads) out[base + i] = (int32_t)sm[i];
 }
 
 // Bounding boxes of the blocks of 32 rows: a warp per 32 positions, for the
@@ -637,9 +633,9 @@ int launch_block_order(const float4 *rows, int dp4, int d, const float4 *reps,
   if (n == 0) return KNN_OK;
   const unsigned blocks = (unsigned)((n + kOrderRun - 1) / kOrderRun);
   if (dp4 == 1)
-    block_order_kernel<1><<<blocks, kOrderRun / 2, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
+    block_order_kernel<1><<<blocks, kOrderThreads, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
   else
-    block_order_kernel<2><<<blocks, kOrderRun / 2, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
+    block_order_kernel<2><<<blocks, kOrderThreads, 0, s>>>(rows, d, reps, skeys, off, perm, n, out);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }

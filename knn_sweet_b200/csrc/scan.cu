@@ -678,7 +678,8 @@ constexpr int scan_min_blocks() {
   return ((DP4 == 0 || DP4 >= 4) ? KNN_TARGET_WARPS_WIDE : KNN_TARGET_WARPS) / WARPS;
 }
 
-template <int DP4, bool IDXROW, int L, int WARPS>
+// ONE: the reference set is a single cluster of narrow rows (small joins).
+template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     scan_kernel(const ScanArgs a) {
   using TK = TopKFor<L>;
@@ -734,8 +735,9 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     } else {
       slot += a.slot_base;
     }
-    const int64_t q = a.qorder[slot];
-    const int qc = a.slot_cl[slot];
+    // (one cluster, queries in their own order: no slot arrays)
+    const int64_t q = a.qorder ? a.qorder[slot] : slot;
+    const int qc = a.slot_cl ? a.slot_cl[slot] : 0;
     if (lane == 0) {
       unsigned *sw = tk.stat();
       sw[kSideSlot] = (unsigned)slot;
@@ -917,29 +919,61 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const int n_c = __shfl_sync(kFull, cnn, src);
         if constexpr (kBlocks) {
           // a lane per block of 32 members: the blocks whose box comes within
-          // the threshold, in order, as long as they still do
+          // the threshold.  In a cluster of a list they come in order (taking
+          // the nearest first cost more than it saved on the k = 200 self-join:
+          // 3.40 -> 3.57 ms); ONE cluster without a starting bound needs its
+          // nearest first
           const int nblk = (n_c + 31) >> 5;
           const int64_t slot0 =
               a.boxes ? block_slot(start, __shfl_sync(kFull, rs, src)) : 0;
-          for (int b0 = 0; b0 < nblk; b0 += 32) {
-            float bd = b0 + lane < nblk ? 0.0f : __int_as_float(0x7f800000);
-            if (a.boxes && b0 + lane < nblk) {
-              float4 lo[DP4], hi[DP4];
-              const float4 *b = a.boxes + (slot0 + b0 + lane) * 2 * DP4;
+          // (distance words; all ones: no block)
+          auto box_of = [&](int blk) -> uint32_t {
+            if (blk >= nblk) return 0xffffffffu;
+            if (!a.boxes) return 0u;
+            float4 lo[DP4], hi[DP4];
+            const float4 *b = a.boxes + (slot0 + blk) * 2 * DP4;
 #pragma unroll
-              for (int e = 0; e < DP4; e++) {
-                lo[e] = b[e];
-                hi[e] = b[DP4 + e];
-              }
-              bd = box_dist2<DP4>(qr.v, lo, hi);
+            for (int e = 0; e < DP4; e++) {
+              lo[e] = b[e];
+              hi[e] = b[DP4 + e];
             }
-            unsigned todo = __ballot_sync(kFull, b0 + lane < nblk && !(bd > tk.thr_d2));
-            while (todo) {
-              const int t = __ffs((int)todo) - 1;
-              todo &= todo - 1;
-              if (__shfl_sync(kFull, bd, t) > tk.thr_d2) continue;
-              const int p = 32 * (b0 + t) + lane;
-              step(start, p, p < n_c);
+            return __float_as_uint(box_dist2<DP4>(qr.v, lo, hi));
+          };
+          if constexpr (ONE) {
+            // the 32 blocks with the nearest one among them to begin with
+            const int rounds = (nblk + 31) >> 5;
+            int b0 = 0;
+            uint32_t best = 0xffffffffu;
+            for (int t = 0; rounds > 1 && t < rounds; t++) {
+              const uint32_t m = __reduce_min_sync(kFull, box_of(32 * t + lane));
+              if (m < best) {
+                best = m;
+                b0 = 32 * t;
+              }
+            }
+            for (int t = 0; t < rounds; t++, b0 = b0 + 32 < 32 * rounds ? b0 + 32 : 0) {
+              uint32_t bd = box_of(b0 + lane);
+              for (;;) {
+                const uint32_t next = __reduce_min_sync(kFull, bd);
+                if (next == 0xffffffffu || __uint_as_float(next) > tk.thr_d2) break;
+                const int at = __ffs((int)__ballot_sync(kFull, bd == next)) - 1;
+                if (lane == at) bd = 0xffffffffu;
+                const int p = 32 * (b0 + at) + lane;
+                step(start, p, p < n_c);
+              }
+            }
+          } else {
+            for (int b0 = 0; b0 < nblk; b0 += 32) {
+              const uint32_t bw = box_of(b0 + lane);
+              const float bd = __uint_as_float(bw);
+              unsigned todo = __ballot_sync(kFull, bw != 0xffffffffu && !(bd > tk.thr_d2));
+              while (todo) {
+                const int t = __ffs((int)todo) - 1;
+                todo &= todo - 1;
+                if (__shfl_sync(kFull, bd, t) > tk.thr_d2) continue;
+                const int p = 32 * (b0 + t) + lane;
+                step(start, p, p < n_c);
+              }
             }
           }
           continue;
@@ -1027,12 +1061,12 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
 // clusters: 43 -> 104), hence 4 there.
 static int split_waves(int Rs) { return Rs >= 256 ? 8 : 4; }
 
-template <int DP4, bool IDXROW, int L, int WARPS>
+template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
   using TK = TopKFor<L>;
   const size_t smem = (size_t)WARPS * TK::kSmemKeys * sizeof(uint64_t) +
                       (DP4 > 0 ? 0 : (size_t)WARPS * a.dp4 * sizeof(float4));
-  auto kern = scan_kernel<DP4, IDXROW, L, WARPS>;
+  auto kern = scan_kernel<DP4, IDXROW, L, WARPS, ONE>;
   if (smem > 48 * 1024)
     KNN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
@@ -1050,14 +1084,20 @@ static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
   return KNN_OK;
 }
 
-template <int DP4, bool IDXROW>
+template <int DP4, bool IDXROW, bool ONE>
 static int launch_scan_l(const ScanArgs &a, int num_sms, cudaStream_t s) {
-  if (a.k <= KNN_REG_TOPK_MAX_K) return launch_scan_t<DP4, IDXROW, 32, 8>(a, num_sms, s);
-  if (a.k <= 64) return launch_scan_t<DP4, IDXROW, 64, 8>(a, num_sms, s);
-  if (a.k <= 128) return launch_scan_t<DP4, IDXROW, 128, 8>(a, num_sms, s);
-  if (a.k <= 256) return launch_scan_t<DP4, IDXROW, 256, 8>(a, num_sms, s);
-  if (a.k <= 512) return launch_scan_t<DP4, IDXROW, 512, 4>(a, num_sms, s);
-  return launch_scan_t<DP4, IDXROW, 1024, 4>(a, num_sms, s);
+  if (a.k <= KNN_REG_TOPK_MAX_K) return launch_scan_t<DP4, IDXROW, 32, 8, ONE>(a, num_sms, s);
+  if (a.k <= 64) return launch_scan_t<DP4, IDXROW, 64, 8, ONE>(a, num_sms, s);
+  if (a.k <= 128) return launch_scan_t<DP4, IDXROW, 128, 8, ONE>(a, num_sms, s);
+  if (a.k <= 256) return launch_scan_t<DP4, IDXROW, 256, 8, ONE>(a, num_sms, s);
+  if (a.k <= 512) return launch_scan_t<DP4, IDXROW, 512, 4, ONE>(a, num_sms, s);
+  return launch_scan_t<DP4, IDXROW, 1024, 4, ONE>(a, num_sms, s);
+}
+
+template <int DP4, bool IDXROW>
+static int launch_scan_n(const ScanArgs &a, int num_sms, cudaStream_t s) {
+  return a.Rs == 1 ? launch_scan_l<DP4, IDXROW, true>(a, num_sms, s)
+                   : launch_scan_l<DP4, IDXROW, false>(a, num_sms, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1714,8 +1754,8 @@ __global__ void __launch_bounds__(kBandThreads) band_resolve_kernel(const ScanAr
   unsigned long long evals = 0;
   for (unsigned u = blockIdx.x; u < total; u += gridDim.x) {
     const int32_t slot = a.unres_slot[u];
-    const int64_t q = a.qorder[slot];
-    const int qc = a.slot_cl[slot];
+    const int64_t q = a.qorder ? a.qorder[slot] : slot;
+    const int qc = a.slot_cl ? a.slot_cl[slot] : 0;
     int32_t *oi = a.out_idx + q * k;
     float *od = a.out_dist + q * k;
     __syncthreads();  // the previous query is done with the shared state
@@ -1878,7 +1918,7 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
   // 100,000 395 / 635, 10^6 2220 / 8271; k = 1: 10,000 61 / 51, 16,000 70 / 74,
   // 32,000 84 / 137; k = 32: 50,000 301 / 336.
   const int64_t fill = (int64_t)num_sms * 32 * (a.k == 1 ? 3 : 8);
-  if (a.k <= 32 && a.m >= fill && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
+  if (a.k <= 32 && a.m >= fill && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
       return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)
                           : launch_group_scan<1, false>(a, num_sms, s);
@@ -1886,13 +1926,13 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
                         : launch_group_scan<2, false>(a, num_sms, s);
   }
   switch (a.dp4_tmpl) {
-    case 1: return a.idx_in_row ? launch_scan_l<1, true>(a, num_sms, s)
-                                : launch_scan_l<1, false>(a, num_sms, s);
-    case 2: return a.idx_in_row ? launch_scan_l<2, true>(a, num_sms, s)
-                                : launch_scan_l<2, false>(a, num_sms, s);
-    case 4: return launch_scan_l<4, false>(a, num_sms, s);
-    case 8: return launch_scan_l<8, false>(a, num_sms, s);
-    default: return launch_scan_l<0, false>(a, num_sms, s);
+    case 1: return a.idx_in_row ? launch_scan_n<1, true>(a, num_sms, s)
+                                : launch_scan_n<1, false>(a, num_sms, s);
+    case 2: return a.idx_in_row ? launch_scan_n<2, true>(a, num_sms, s)
+                                : launch_scan_n<2, false>(a, num_sms, s);
+    case 4: return launch_scan_l<4, false, false>(a, num_sms, s);
+    case 8: return launch_scan_l<8, false, false>(a, num_sms, s);
+    default: return launch_scan_l<0, false, false>(a, num_sms, s);
   }
 }
 

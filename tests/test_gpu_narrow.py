@@ -70,3 +70,25 @@ def test_tiny_clusters_and_far_outliers(cuda_device, oracle):
     q = rng.standard_normal((MANY, 3)).astype(np.float32)
     _check(oracle, q, r, 8, sreps=500)
     _check(oracle, q, r, 8, sreps=1, qreps=1)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 1024, 1025, 4095, 4096, 4097])
+@pytest.mark.parametrize("d,k", [(1, 5), (3, 16), (3, 200), (4, 1), (5, 33), (8, 24)])
+def test_small_joins(cuda_device, oracle, n, d, k):
+    # up to 4,096 reference rows and no representatives asked for: one cluster
+    rng = np.random.default_rng(1000 * d + n)
+    r = rng.standard_normal((n, d)).astype(np.float32)
+    q = (2 * rng.standard_normal((123, d))).astype(np.float32)
+    _check(oracle, q, r, k, sample=123)
+    _check(oracle, r, r, k, sample=200)
+    ints = rng.integers(0, 6, (n, d)).astype(np.float32)
+    _check(oracle, ints, ints, k, exact=True, sample=100)
+
+
+def test_small_join_self_and_missing_slots(cuda_device):
+    import torch
+    x = torch.tensor([[0.0, 0, 0], [1, 0, 0], [float("nan"), 0, 0], [3, 0, 0]], device="cuda")
+    idx, dist = knnjoin(x, None, 6)
+    assert idx[0].tolist() == [0, 1, 3, -1, -1, -1]
+    assert dist[0, :3].tolist() == [0.0, 1.0, 3.0] and bool(torch.isinf(dist[0, 3:]).all())
+    assert idx[2].tolist() == [-1] * 6  # no distance from a NaN query is a number
