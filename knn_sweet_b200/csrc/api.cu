@@ -222,13 +222,13 @@ int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d,
   // nearest representative (BF16 tensor-core arg-min + exact FP32 distance to
   // the winner for d >= 16, FP32 CUDA cores otherwise), then one sort into
   // clusters
-  auto cluster = [&](const float4 *x, int64_t cnt) -> int {
+  auto cluster = [&](const float4 *x, int64_t cnt, int dist_bits) -> int {
     if (tc_assign)
       KNN_TRY(launch_assign_tc(x, cnt, dp4s, d, cs->reps, R, tc_scratch, cl, dr, err, s));
     else
       KNN_TRY(launch_assign(x, cnt, dp4s, cs->reps, R, cl, dr, s));
     KNN_TRY(launch_cluster_sort(cl, dr, cnt, R, keys, vals, cs->skeys, cs->perm, temp,
-                                temp_bytes, s));
+                                temp_bytes, s, dist_bits));
     return launch_cluster_offsets(cs->skeys, cnt, R, cs->off, s);
   };
   // Lloyd steps: the representatives move to their clusters' centroids (the
@@ -253,13 +253,18 @@ int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d,
       KNN_TRY(launch_sample_rows(rows, dp4s, stride, cnt, seed, sample, s));
       x = sample;
     }
+    uint64_t *split;
+    KNN_TRY(ar.alloc(&split, split_scratch_words(R)));
+    KNN_CUDA_TRY(cudaMemsetAsync(split, 0, sizeof(uint64_t), s));
     for (int it = 0; it < lloyd_iters; it++) {
-      KNN_TRY(cluster(x, cnt));
+      // (twelve bits of the distance tell the far members of a cluster)
+      KNN_TRY(cluster(x, cnt, 12));
       KNN_TRY(launch_centroids(x, dp4s, cs->perm, cs->off, R, cs->reps, s));
-      KNN_TRY(launch_split_clusters(x, dp4s, cs->perm, cs->off, cs->skeys, R, cs->reps, s));
+      KNN_TRY(launch_split_clusters(x, dp4s, cs->perm, cs->off, cs->skeys, R, split,
+                                    cs->reps, s));
     }
   }
-  KNN_TRY(cluster(rows, n));
+  KNN_TRY(cluster(rows, n, 32));
   return KNN_OK;
 }
 
@@ -495,6 +500,9 @@ int build_query_side(const RefSide &R, bool share, const float *q, int64_t m, in
   return KNN_OK;
 }
 
+// Queries from which on the clusters are searched in the order of their reach.
+constexpr int64_t kOrderedQueries = 8192;
+
 // The search of the query clusters c0 .. c1-1, whose slots are
 // slot0 .. slot0+nslot-1: the BF16 tile search (precision BF16_REFINE) and
 // the FP32 scan, results into rows of out_idx / out_dist (query order).
@@ -511,6 +519,15 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   KNN_CUDA_TRY(cudaGetDevice(&dev));
   KNN_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
   const int nclu = c1 - c0;
+
+  // wide rows and many queries: the query clusters that reach farthest first
+  const bool whole = slot0 == 0 && nslot == m;
+  int32_t *corder = nullptr, *cstart = nullptr;
+  if (whole && R.col_blocks && m >= kOrderedQueries) {
+    KNN_TRY(ar.alloc(&corder, (size_t)nclu));
+    KNN_TRY(ar.alloc(&cstart, (size_t)nclu));
+    KNN_TRY(launch_cluster_order(Q.rlen, Q.qset.off, nclu, corder, cstart, s));
+  }
 
   // BF16+refine form: tensor-core tiles over the same candidate lists; the
   // FP32 scan below then runs only for the queries the tiles hand back.
@@ -532,7 +549,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
     KNN_TRY(ar.alloc(&buf_lu, slots));
     KNN_TRY(ar.alloc(&buf_pos, slots));
     KNN_TRY(ar.alloc(&fb_slots, (size_t)nslot));
-    KNN_TRY(launch_tile_list(Q.qset.off + c0, nclu, c0, tile_list, ntiles, s));
+    KNN_TRY(launch_tile_list(Q.qset.off + c0, nclu, c0, corder, tile_list, ntiles, s));
     TileArgs t{};
     t.qrows = Q.Qp;
     t.dp4 = dp4s;
@@ -613,6 +630,10 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   a.out_dist = out_dist;
   KNN_TRY(ar.alloc(&a.unres_slot, (size_t)nslot));
   a.unres_count = reinterpret_cast<unsigned *>(ctr + kCtrUnres);
+  if (R.col_blocks) {
+    KNN_TRY(ar.alloc(&a.far_slot, (size_t)kFarQueries));
+    KNN_TRY(ar.alloc(&a.far_count, 1));
+  }
   a.work_counter = ctr + kCtrWork;
   a.counters = ctr + kCtrScan;
   if (tiles) {
@@ -626,7 +647,6 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   // chunks, 8.18 with 24, 8.17 with 32; the copy alone takes 6.89 ms), the
   // first one small (8.23 -> 8.10 ms on a box whose copy takes 7.15 ms)
   const int64_t out_bytes = m * (int64_t)k * 8;
-  const bool whole = slot0 == 0 && nslot == m;
   const int nchunks =
       (sink && whole && !tiles && out_bytes >= (16 << 20) && m >= 8 * 1024)
           ? (int)std::min<int64_t>(32, std::max<int64_t>(8, out_bytes >> 24))
@@ -684,6 +704,15 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
     }
     sink->done = true;
   } else {
+    if (corder && !tiles) {
+      int32_t *order;
+      unsigned *count;
+      KNN_TRY(ar.alloc(&order, (size_t)m));
+      KNN_TRY(ar.alloc(&count, 1));
+      KNN_TRY(launch_slot_order(Q.slot_cl, Q.qset.off, cstart, m, order, count, s));
+      a.slot_list = order;
+      a.slot_count = count;
+    }
     KNN_TRY(launch_scan(a, num_sms, s));
   }
   return KNN_OK;

@@ -39,25 +39,29 @@ constexpr int kTileN = 256;  // representatives per MMA (TMEM columns)
 // each); the points carry -0.5 there, so the MMA yields p.r - |r|^2 / 2 and
 // the nearest representative is its arg-max.  Padding rows carry the largest
 // finite BF16 value as the norm: they never win.
-__global__ void reps_to_bf16_tiles_kernel(const float4 *__restrict__ reps, int R, int dp4,
-                                          int d, int KD, int Rpad,
-                                          __nv_bfloat16 *__restrict__ tiles) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= Rpad) return;
+// A warp per representative, a lane per 8 columns (one thread per
+// representative took 18 us at d = 128, this 3 to 5).
+__global__ void __launch_bounds__(256)
+    reps_to_bf16_tiles_kernel(const float4 *__restrict__ reps, int R, int dp4, int d, int KD,
+                              int Rpad, __nv_bfloat16 *__restrict__ tiles) {
+  const int lane = threadIdx.x & 31;
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (r >= Rpad) return;  // whole warps
   unsigned char *tile = reinterpret_cast<unsigned char *>(tiles) +
                         (size_t)(r / kTileN) * tc::tile_bytes(kTileN, KD);
   const int rr = r % kTileN;
   auto coord = [&](int k) -> float {
-    const float4 c = reps[(size_t)r * dp4 + (k >> 2)];
-    return (k & 3) == 0 ? c.x : (k & 3) == 1 ? c.y : (k & 3) == 2 ? c.z : c.w;
+    return r < R && k < d ? reinterpret_cast<const float *>(reps + (size_t)r * dp4)[k] : 0.0f;
   };
+  float nrm = 0.0f;
+  for (int k = lane; k < d; k += 32) {
+    const float xr = __bfloat162float(__float2bfloat16_rn(coord(k)));
+    nrm = __fmaf_rn(xr, xr, nrm);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(kFull, nrm, o);
   __nv_bfloat16 part[3];
   if (r < R) {
-    float nrm = 0.0f;
-    for (int k = 0; k < d; k++) {
-      const float xr = __bfloat162float(__float2bfloat16_rn(coord(k)));
-      nrm = __fmaf_rn(xr, xr, nrm);
-    }
     // each remainder is exact in FP32: the part is the remainder rounded
 #pragma unroll
     for (int t = 0; t < 3; t++) {
@@ -68,14 +72,15 @@ __global__ void reps_to_bf16_tiles_kernel(const float4 *__restrict__ reps, int R
     part[0] = __ushort_as_bfloat16(0x7f7f);
     part[1] = part[2] = __float2bfloat16_rn(0.0f);
   }
-  for (int k0 = 0; k0 < KD; k0 += 8) {
+  for (int k0 = 8 * lane; k0 < KD; k0 += 256) {
     __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
       const int k = k0 + e;
-      v[e] = k >= d && k < d + 3 ? part[k - d]
-             : (r < R && k < d)  ? __float2bfloat16_rn(coord(k))
-                                 : __float2bfloat16_rn(0.0f);
+      v[e] = k == d       ? part[0]
+             : k == d + 1 ? part[1]
+             : k == d + 2 ? part[2]
+                          : __float2bfloat16_rn(coord(k));
     }
     *reinterpret_cast<uint4 *>(tile + tc::tile_offset(rr, k0, KD)) =
         *reinterpret_cast<const uint4 *>(v);
@@ -324,7 +329,7 @@ int launch_assign_tc(const float4 *rows, int64_t n, int dp4, int d, const float4
   const int KD = assign_kd(d);
   const int Rpad = (R + kTileN - 1) / kTileN * kTileN;
   __nv_bfloat16 *tiles = static_cast<__nv_bfloat16 *>(scratch);
-  reps_to_bf16_tiles_kernel<<<(Rpad + 127) / 128, 128, 0, s>>>(reps, R, dp4, d, KD, Rpad, tiles);
+  reps_to_bf16_tiles_kernel<<<(Rpad + 7) / 8, 256, 0, s>>>(reps, R, dp4, d, KD, Rpad, tiles);
   KNN_LAUNCH_CHECK();
   // representative tiles of 128 rows: a CTA then holds 256 TMEM columns and
   // two CTAs share an SM (measured faster than 256-row tiles with one CTA

@@ -24,6 +24,11 @@ namespace knnsweet {
 //     (the host std::sort of knnjoin.cu:1080-1091); only the survivors
 //     enter the sort.
 // ---------------------------------------------------------------------------
+// The bisection stops this many representable values above the exact k-th: a
+// bound 2.4e-4 wider prunes as well and takes half the counting rounds
+// (8,192 by 8,192 clusters: 2.25 ms with the exact value, 1.68 so).
+constexpr unsigned kBoundUlps = 2048;
+
 // One query cluster's bound and candidate list, by one block.  The reference
 // clusters are the Rs_loc consecutive clusters whose offsets start at soff
 // (soff[0] .. soff[Rs_loc]; their points are sdist[soff[j] ..]); dq[j] is the
@@ -96,7 +101,7 @@ static __device__ __forceinline__ void bounds_filter_block(const float *dq, int 
   // smallest bit pattern T with count(values <= T) >= kk; count(hi) >= kk.
   // lo: the smallest value of all (nothing lies below it), lo <= hi
   // invariant: answer in [lo, hi]
-  while (lo < hi) {
+  while (hi - lo > kBoundUlps) {
     unsigned mid = lo + ((hi - lo) >> 1);
     float T = __uint_as_float(mid);
     int cnt = 0;
@@ -240,7 +245,7 @@ static __device__ __forceinline__ void bounds_filter_warp(
   if (u < hi) hi = u;
   __syncwarp();
   // smallest bit pattern T with count(values <= T) >= kk, in [lo, hi]
-  while (lo < hi) {
+  while (hi - lo > kBoundUlps) {
     const unsigned mid = lo + ((hi - lo) >> 1);
     const float T = __uint_as_float(mid);
     int cnt = 0;

@@ -262,10 +262,10 @@ __device__ __forceinline__ int warp_lower_bound_coarse(const float *__restrict__
 // E t + e in x[e] of thread t; blockDim.x a power of two, at least 32): a
 // bitonic network whose strides inside a thread and inside a warp stay in
 // registers, so that only strides of 32 E keys or more go through shared
-// memory (sm: E * blockDim.x words) -- 6 of 55 stages for 1,024 keys in 256
+// memory (sm: E * blockDim.x keys) -- 6 of 55 stages for 1,024 keys in 256
 // threads.  Every thread of the block calls it.
-template <int E>
-__device__ __forceinline__ void block_sort_u32(uint32_t (&x)[E], uint32_t *sm) {
+template <int E, class T>
+__device__ __forceinline__ void block_sort(T (&x)[E], T *sm) {
   const int t = threadIdx.x, total = E * blockDim.x;
   for (int size = 2; size <= total; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -276,7 +276,7 @@ __device__ __forceinline__ void block_sort_u32(uint32_t (&x)[E], uint32_t *sm) {
           for (int f = 1; f < E; f <<= 1)
             if (stride == f && (e & f) == 0) {
               const bool up = ((E * t + e) & size) == 0;
-              const uint32_t lo = min(x[e], x[e | f]), hi = max(x[e], x[e | f]);
+              const T lo = min(x[e], x[e | f]), hi = max(x[e], x[e | f]);
               x[e] = up ? lo : hi;
               x[e | f] = up ? hi : lo;
             }
@@ -293,7 +293,7 @@ __device__ __forceinline__ void block_sort_u32(uint32_t (&x)[E], uint32_t *sm) {
 #pragma unroll
       for (int e = 0; e < E; e++) {
         const int i = E * t + e;
-        const uint32_t o = shared ? sm[i ^ stride] : __shfl_xor_sync(kFull, x[e], stride / E);
+        const T o = shared ? sm[i ^ stride] : __shfl_xor_sync(kFull, x[e], stride / E);
         const bool least = ((i & stride) == 0) == ((i & size) == 0);
         x[e] = least ? min(x[e], o) : max(x[e], o);
       }

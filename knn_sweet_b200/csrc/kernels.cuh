@@ -19,6 +19,8 @@ namespace knnsweet {
 constexpr int kScanCounters = 7;
 
 // Arguments of the per-query scan.
+constexpr unsigned kFarQueries = 4096;
+
 struct ScanArgs {
   const float4 *qrows;      // m x dp4, original query order
   const int32_t *qorder;    // slot -> query row (grouped by query cluster)
@@ -59,6 +61,9 @@ struct ScanArgs {
   const int32_t *slot_list;    // optional: scan only these slots ...
   const unsigned *slot_count;  // ... *slot_count of them (device count);
   int split_max;               // a block per query up to this many (launch_scan)
+  int32_t *far_slot;           // optional (wide rows): room for kFarQueries slots,
+  unsigned *far_count;         // and their number: queries the scan gave up on,
+                               // which get a block each afterwards
   int64_t slot_base;           // without a list: slots slot_base .. + m - 1
   int Rs;
   int64_t n_ref;            // reference points (0: unknown); with Rs it gives
@@ -77,6 +82,12 @@ struct ScanArgs {
   unsigned long long *counters;      // kScanCounters statistics (or null)
 };
 
+// The query clusters by the length of their candidate lists, longest first
+// (Rq <= KNN_MAX_REPS), and the slots in that order of their clusters.
+int launch_cluster_order(const int32_t *rlen, const int32_t *qoff, int Rq, int32_t *corder,
+                         int32_t *cstart, cudaStream_t s);
+int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t *cstart,
+                      int64_t m, int32_t *order, unsigned *count, cudaStream_t s);
 int launch_pack_rows(const float *src, int64_t n, int d, int dp4, float4 *dst,
                      cudaStream_t s);
 // Raises *inexact unless every value of x[0..count) is an integer small enough
@@ -104,12 +115,16 @@ int launch_sample_rows(const float4 *rows, int dp4, int64_t stride, int64_t cnt,
                        float4 *out, cudaStream_t s);
 int launch_centroids(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off, int R,
                      float4 *reps, cudaStream_t s);
+size_t split_scratch_words(int R);
 int launch_split_clusters(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off,
-                          const uint64_t *skeys, int R, float4 *reps, cudaStream_t s);
+                          const uint64_t *skeys, int R, uint64_t *scratch, float4 *reps,
+                          cudaStream_t s);
+// Sorts (cluster, distance) keys; dist_bits < 32 orders the distances by
+// their upper bits only.
 int launch_cluster_sort(const int32_t *cl, const float *dr, int64_t n, int R,
                         uint64_t *keys, int32_t *vals, uint64_t *skeys,
                         int32_t *perm, void *temp, size_t temp_bytes,
-                        cudaStream_t s);
+                        cudaStream_t s, int dist_bits = 32);
 size_t chunk_slots_temp_bytes(int64_t m, int nchunks);
 int launch_chunk_slots(const int32_t *qorder, int64_t m, int first, int chunk_rows, int nchunks,
                        uint32_t *keys, uint32_t *keys_out, int32_t *vals, int32_t *slots,
@@ -199,8 +214,9 @@ int tile_search_geometry(int d, int k, int margin, int num_sms, int *grid, int *
                          size_t *smem);
 // Tiles of the query clusters c_base .. c_base + Rq - 1 (qoff points at
 // c_base's offset; the tiles carry absolute cluster ids and slots).
-int launch_tile_list(const int32_t *qoff, int Rq, int c_base, int32_t *tiles, int32_t *ntiles,
-                     cudaStream_t s);
+// corder (or null): the clusters in the order their tiles are wanted.
+int launch_tile_list(const int32_t *qoff, int Rq, int c_base, const int32_t *corder,
+                     int32_t *tiles, int32_t *ntiles, cudaStream_t s);
 int launch_tile_search(const TileArgs &a, int grid, size_t smem, cudaStream_t s);
 
 // The calling thread's two streams for host-buffer calls (cached per device,

@@ -33,6 +33,7 @@
 // Bounds are widened by a rounding slack (bound_tol) so that FP32 rounding
 // never prunes a point that the FP32 distances would rank in the top k.
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -678,6 +679,13 @@ constexpr int scan_min_blocks() {
   return ((DP4 == 0 || DP4 >= 4) ? KNN_TARGET_WARPS_WIDE : KNN_TARGET_WARPS) / WARPS;
 }
 
+// Steps of 32 members after which a warp leaves its query of wide rows to a
+// whole block (a launch behind the scan's): a few queries between distant
+// groups of points reach a hundred times the members of the others, and the
+// scan took as long as the longest (N = 10^6, d = 32, k = 32, six data sets:
+// 2.9 to 5.5 ms, 2.9 to 3.3 with this).
+constexpr int kFarSteps = 512;
+
 // ONE: the reference set is a single cluster of narrow rows (small joins).
 template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
@@ -710,9 +718,10 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
   // threshold (s_thr, distance bits), and warp 0 merges their candidates
   __shared__ unsigned s_thr;
   __shared__ long long s_slot;
-  const bool split =
-      kWideRows &&
-      (a.slot_list ? (int64_t)*a.slot_count : a.m) <= (int64_t)a.split_max;
+  // (more may have been counted than there was room for in the far list)
+  const int64_t listed =
+      a.slot_list ? min((int64_t)*a.slot_count, a.m) : a.m;
+  const bool split = kWideRows && listed <= (int64_t)a.split_max;
   for (;;) {
     long long slot = 0;
     if (split) {
@@ -728,7 +737,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       slot = __shfl_sync(kFull, slot, 0);
     }
     if (a.slot_list) {
-      if (slot >= (long long)*a.slot_count) break;
+      if (slot >= listed) break;
       slot = a.slot_list[slot];
     } else if (slot >= a.m) {
       break;
@@ -758,7 +767,10 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     // one step: lane's member p of the cluster at `start`, if `in`.  Row
     // indices fit 32 bits (the result indices are int32): unsigned offsets make
     // every address one wide multiply-add
+    int steps = 0;      // (wide rows: how far the query has come ...
+    bool far = false;   // ... and whether it is left to a whole block)
     auto step = [&](int start, int p, bool in) {
+      if constexpr (kWideRows) steps++;
       const unsigned gp = (unsigned)(start + p);
       float v = 0.0f;
       int32_t idx = 0;
@@ -914,6 +926,17 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           tk.count(kStatPruned, 1, lane);
           continue;
         }
+        if (kWideRows && steps > kFarSteps && a.far_slot && !split) {
+          unsigned at = 0;
+          if (lane == 0) at = atomicAdd(a.far_count, 1u);
+          at = __shfl_sync(kFull, at, 0);
+          if (at < kFarQueries) {
+            if (lane == 0) a.far_slot[at] = (int32_t)slot;
+            far = true;
+            break;
+          }
+          steps = -(1 << 30);  // no room: the warp carries on
+        }
         tk.count(kStatVisited, 1, lane);
         const int start = __shfl_sync(kFull, cst, src);
         const int n_c = __shfl_sync(kFull, cnn, src);
@@ -996,6 +1019,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           if (__shfl_sync(kFull, ds > hi_v, 31)) break;
         }
       }
+      if (kWideRows && far) break;
     }
     tk.finish(lane, a.d);
     if (split) {
@@ -1022,7 +1046,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       }
     }
     __syncwarp();
-    if (!split || w == 0) {
+    if ((!split || w == 0) && !far) {
       const unsigned *sw = tk.stat();
       const int32_t e_slot = (int32_t)sw[kSideSlot];
       const int64_t e_q = (int64_t)sw[kSideQuery];
@@ -1055,11 +1079,11 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
 // Queries of wide rows up to this many times the resident blocks get a block
 // each (scan_kernel's split): a warp per query then leaves the chip waiting
 // for the query with the most clusters to visit.  200,003 reference rows,
-// d = 17, k = 10, 1,013 queries: search 971 -> 289 us; 100 queries 746 -> 141;
-// 100,000 rows, d = 64, 2,000 queries (8 times): 2430 -> 1526.  With short
-// lists the blocks' own start and merge weigh more (2,000 queries over 72
-// clusters: 43 -> 104), hence 4 there.
-static int split_waves(int Rs) { return Rs >= 256 ? 8 : 4; }
+// d = 17, k = 10, 1,013 queries: search 971 -> 289 us; 100 queries 746 -> 141.
+// With more queries the chip is full either way, and every warp of a block
+// starts without a threshold: eight times instead of four gave 2,000 queries
+// of d = 64 1526 us for 2430, but 2,000 of d = 32 and k = 32 760 for 225.
+constexpr int kSplitWaves = 4;
 
 template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
@@ -1075,7 +1099,8 @@ static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
   if (per_sm < 1) per_sm = 1;
   int64_t grid = (int64_t)num_sms * per_sm;
   ScanArgs b = a;
-  b.split_max = (int)(split_waves(a.Rs) * grid);
+  // (the queries left by a first launch are always split)
+  b.split_max = a.split_max > 0 ? a.split_max : (int)(kSplitWaves * grid);
   const int64_t want = a.m <= b.split_max ? a.m : (a.m + WARPS - 1) / WARPS;
   if (grid > want) grid = want;
   if (grid < 1) grid = 1;
@@ -1905,7 +1930,18 @@ int launch_scan(const ScanArgs &a, int num_sms, cudaStream_t s) {
     return KNN_EINTERNAL;
   }
   KNN_CUDA_TRY(cudaMemsetAsync(a.unres_count, 0, sizeof(unsigned), s));
-  const int rc = launch_scan_kernels(a, num_sms, s);
+  if (a.far_slot) KNN_CUDA_TRY(cudaMemsetAsync(a.far_count, 0, sizeof(unsigned), s));
+  int rc = launch_scan_kernels(a, num_sms, s);
+  if (rc == KNN_OK && a.far_slot) {
+    ScanArgs f = a;
+    f.slot_list = a.far_slot;
+    f.slot_count = a.far_count;
+    f.far_slot = nullptr;
+    f.m = std::min<int64_t>(a.m, kFarQueries);
+    f.split_max = INT_MAX;
+    KNN_CUDA_TRY(cudaMemsetAsync(a.work_counter, 0, sizeof(unsigned long long), s));
+    rc = launch_scan_kernels(f, num_sms, s);
+  }
   if (rc != KNN_OK) return rc;
   return launch_band_resolve(a, num_sms, s);
 }

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kPrepThreads)
     uint32_t x[E];
 #pragma unroll
     for (int e = 0; e < E; e++) x[e] = key_of(e * kPrepThreads + tid);
-    block_sort_u32<E>(x, key);
+    block_sort(x, key);
     __syncthreads();
 #pragma unroll
     for (int e = 0; e < E; e++) key[E * tid + e] = x[e];

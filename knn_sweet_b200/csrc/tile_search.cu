@@ -95,13 +95,17 @@ constexpr int kTN = 128;  // member rows per chunk: TMEM columns
 // representative.  One block of 1024 threads, each owning a run of clusters.
 __global__ void __launch_bounds__(1024)
     tile_list_kernel(const int32_t *__restrict__ qoff, int Rq, int c_base,
+                     const int32_t *__restrict__ corder,
                      int32_t *__restrict__ tiles, int32_t *__restrict__ ntiles) {
   __shared__ int wsum[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int per = (Rq + 1023) / 1024;
   const int c0 = min(Rq, tid * per), c1 = min(Rq, c0 + per);
   int local = 0;
-  for (int c = c0; c < c1; c++) local += (qoff[c + 1] - qoff[c] + kTM - 1) / kTM;
+  for (int i = c0; i < c1; i++) {
+    const int c = corder ? corder[i] : i;
+    local += (qoff[c + 1] - qoff[c] + kTM - 1) / kTM;
+  }
   int incl = local;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -122,7 +126,8 @@ __global__ void __launch_bounds__(1024)
   }
   __syncthreads();
   int pos = wsum[warp] + incl - local;
-  for (int c = c0; c < c1; c++) {
+  for (int i = c0; i < c1; i++) {
+    const int c = corder ? corder[i] : i;
     const int size = qoff[c + 1] - qoff[c];
     for (int s = 0; s < size; s += kTM) {
       tiles[4 * pos + 0] = c_base + c;
@@ -1020,9 +1025,9 @@ int tile_search_geometry(int d, int k, int margin, int num_sms, int *grid, int *
   return KNN_OK;
 }
 
-int launch_tile_list(const int32_t *qoff, int Rq, int c_base, int32_t *tiles, int32_t *ntiles,
-                     cudaStream_t s) {
-  tile_list_kernel<<<1, 1024, 0, s>>>(qoff, Rq, c_base, tiles, ntiles);
+int launch_tile_list(const int32_t *qoff, int Rq, int c_base, const int32_t *corder,
+                     int32_t *tiles, int32_t *ntiles, cudaStream_t s) {
+  tile_list_kernel<<<1, 1024, 0, s>>>(qoff, Rq, c_base, corder, tiles, ntiles);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }

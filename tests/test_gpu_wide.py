@@ -66,3 +66,17 @@ def test_tile_that_reaches_too_far(cuda_device, oracle):
     oi, od = oracle.bruteforce_f64(q, r, 20)
     assert_matches(idx, dist, oi, od)
     assert st.refine_fallbacks > 0
+
+
+@pytest.mark.parametrize("m", [1500, 5000])
+def test_queries_left_to_a_block(cuda_device, oracle, m):
+    # four clusters of 15,000 rows: every query passes the step limit of a warp
+    # (and, with 5,000, more of them than the list of such queries holds)
+    rng = np.random.default_rng(m)
+    r = rng.standard_normal((60_000, 16)).astype(np.float32)
+    q = rng.standard_normal((m, 16)).astype(np.float32)
+    idx, dist = knnjoin(q, r, 40, sreps=4, qreps=8)
+    rows = rng.permutation(m)[:200]
+    oi, od = oracle.bruteforce_f64(q[rows], r, 40)
+    assert_matches(idx[rows], dist[rows], oi, od)
+    assert (idx >= 0).all()
