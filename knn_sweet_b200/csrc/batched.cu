@@ -29,6 +29,7 @@
 #include "bounds.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "pipeline.cuh"
 
 namespace knnsweet {
 
@@ -269,44 +270,6 @@ __global__ void batched_fill_empty_kernel(int32_t *idx, float *dist, int64_t cou
   }
 }
 
-#define KNN_TRY(expr)              \
-  do {                             \
-    int rc_ = (expr);              \
-    if (rc_ != KNN_OK) return rc_; \
-  } while (0)
-
-// Stream-ordered scratch from the library's per-device pool, released on
-// the same stream when the arena goes out of scope.
-class BatchArena {
- public:
-  explicit BatchArena(cudaStream_t s) : s_(s) {}
-  ~BatchArena() {
-    for (void *p : ptrs_) cudaFreeAsync(p, s_);
-  }
-  BatchArena(const BatchArena &) = delete;
-  BatchArena &operator=(const BatchArena &) = delete;
-  template <class T>
-  int alloc(T **out, size_t count) {
-    *out = nullptr;
-    if (!pool_) KNN_TRY(scratch_pool(&pool_));
-    void *p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, (count ? count : 1) * sizeof(T), pool_, s_);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      set_error("device allocation failed: %s", cudaGetErrorString(e));
-      return e == cudaErrorMemoryAllocation ? KNN_ENOMEM : KNN_ECUDA;
-    }
-    ptrs_.push_back(p);
-    *out = static_cast<T *>(p);
-    return KNN_OK;
-  }
-
- private:
-  cudaStream_t s_;
-  cudaMemPool_t pool_ = nullptr;
-  std::vector<void *> ptrs_;
-};
-
 // Host arrays reach the device as kernel parameters (no pageable copy, so
 // the call stays capturable).
 struct U32Chunk {
@@ -343,7 +306,7 @@ struct BatchSide {
   int32_t *order = nullptr; // slot -> row as the scan takes it (narrow rows: block order)
 };
 
-int cluster_side(BatchArena &ar, const float *pts, const int64_t *off_h, int ncloud, int d,
+int cluster_side(Arena &ar, const float *pts, const int64_t *off_h, int ncloud, int d,
                  int dp4, const std::vector<int32_t> &R_h, uint32_t seed, int trials,
                  cudaStream_t s, BatchSide *b) {
   b->total = off_h[ncloud];
@@ -469,7 +432,7 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
   }
   int rc = KNN_OK;
   {
-    BatchArena ar(s);
+    Arena ar(s);
     unsigned long long *ctr = nullptr;
     auto body = [&]() -> int {
       // [0] scan work counter, [1 ..] scan statistics, then the count of
@@ -692,7 +655,7 @@ int autotune(const float *q, const int64_t *qoff_h, const float *r, const int64_
     }
     float best_a = kAlphaDefault;
     {
-      BatchArena ar(s);
+      Arena ar(s);
       float *sr, *sqp, *od;
       int32_t *oi;
       KNN_TRY(ar.alloc(&sr, (size_t)d * so[ns]));
@@ -829,7 +792,7 @@ extern "C" int knn_join_batched(const float *q, const int64_t *q_offsets, const 
   }
   int rc = KNN_OK;
   {
-    BatchArena ar(s);
+    Arena ar(s);
     float *dq = nullptr, *dr = nullptr, *dd = nullptr;
     int32_t *di = nullptr;
     rc = ar.alloc(&dq, (size_t)m * d);
