@@ -44,8 +44,8 @@ class _KnnDist2(torch.autograd.Function):
         m, d = q.shape
         n = s.shape[0]
         k = idx.shape[1]
+        # (the kernel reads no gradient of a missing neighbour)
         g = grad_d2.contiguous().to(torch.float32)
-        g = torch.where(idx >= 0, g, torch.zeros_like(g))
         grad_q = torch.zeros_like(q)
         grad_s = torch.zeros_like(s) if ctx.needs_input_grad[1] else None
         lib = _lib.load()
@@ -75,16 +75,19 @@ def knn_chamfer(x: torch.Tensor, y: torch.Tensor, k: int = 1) -> torch.Tensor:
     return dxy.sum() + dyx.sum()
 
 
-def _cloud_base(offsets, rows_off, device):
-    """Per query row: the first row of its cloud's reference points.  Built on
-    the device from the per-cloud values (a host-side expansion meant a
-    row-sized pageable copy on every forward pass)."""
+def _cloud_rows(idx, k, q_offsets, r_offsets):
+    """Cloud-relative indices as rows of the concatenated reference points."""
     import numpy as np
-    qo = np.asarray(rows_off, dtype=np.int64)
-    ro = np.asarray(offsets, dtype=np.int64)
-    base = torch.as_tensor(ro[:-1].astype(np.int32)).to(device, non_blocking=True)
-    counts = torch.as_tensor(np.diff(qo)).to(device, non_blocking=True)
-    return torch.repeat_interleave(base, counts, output_size=int(qo[-1]))
+    qo = np.ascontiguousarray(np.asarray(q_offsets, dtype=np.int64))
+    ro = np.ascontiguousarray(np.asarray(r_offsets, dtype=np.int64))
+    out = torch.empty_like(idx)
+    with torch.cuda.device(idx.device):
+        stream = ctypes.c_void_p(torch.cuda.current_stream(idx.device).cuda_stream)
+        rc = _lib.load().knnsweet_cloud_rows(
+            _ptr(idx), ctypes.c_int32(k), qo.ctypes.data_as(ctypes.c_void_p),
+            ro.ctypes.data_as(ctypes.c_void_p), ctypes.c_int32(qo.size - 1), _ptr(out), stream)
+    _lib.check(rc)
+    return out
 
 
 class _KnnDist2Batched(torch.autograd.Function):
@@ -95,8 +98,7 @@ class _KnnDist2Batched(torch.autograd.Function):
         s = sources.detach().contiguous()
         idx, d2 = knnjoin_batched(q, q_offsets, s, r_offsets, k, squared=True)
         # indices relative to each cloud -> rows of the concatenated sources
-        base = _cloud_base(r_offsets, q_offsets, q.device)
-        gidx = torch.where(idx >= 0, idx + base[:, None], idx)
+        gidx = _cloud_rows(idx, k, q_offsets, r_offsets)
         ctx.save_for_backward(q, s, gidx)
         ctx.mark_non_differentiable(idx)
         return d2, idx
@@ -106,8 +108,8 @@ class _KnnDist2Batched(torch.autograd.Function):
         q, s, gidx = ctx.saved_tensors
         m, d = q.shape
         n, k = s.shape[0], gidx.shape[1]
-        g = torch.where(gidx >= 0, grad_d2.contiguous().to(torch.float32),
-                        torch.zeros_like(grad_d2, dtype=torch.float32))
+        # (the kernel reads no gradient of a missing neighbour)
+        g = grad_d2.contiguous().to(torch.float32)
         grad_q = torch.zeros_like(q)
         grad_s = torch.zeros_like(s) if ctx.needs_input_grad[2] else None
         lib = _lib.load()

@@ -828,3 +828,53 @@ extern "C" int knn_join_batched(const float *q, const int64_t *q_offsets, const 
   }
   return rc;
 }
+
+// Cloud-relative neighbour indices -> rows of the concatenated reference
+// points: out[i * k + t] = idx[i * k + t] + r_offsets[cloud of i], -1 kept.  One
+// kernel for the training step, which spent a repeat, an addition, a
+// comparison and a selection over all rows on it (64 pairs, k = 8: 0.2 ms).
+namespace knnsweet {
+namespace {
+__global__ void cloud_rows_kernel(const int32_t *__restrict__ idx, int64_t m, int k,
+                                  const int32_t *__restrict__ qoff,
+                                  const int32_t *__restrict__ roff, int ncloud,
+                                  int32_t *__restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m * k;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t j = idx[i];
+    out[i] = j < 0 ? j : j + roff[cloud_of(qoff, ncloud, i / k)];
+  }
+}
+}  // namespace
+}  // namespace knnsweet
+
+// (not part of the public ABI: the Python training step's own helper)
+extern "C" int knnsweet_cloud_rows(const int32_t *idx, int32_t k, const int64_t *q_offsets,
+                                   const int64_t *r_offsets, int32_t ncloud, int32_t *out,
+                                   void *stream) {
+  error_buffer().clear();
+  if (!q_offsets || !r_offsets || ncloud < 0 || k < 1) {
+    set_error("cloud rows: bad arguments");
+    return KNN_EINVAL;
+  }
+  const int64_t m = q_offsets[ncloud];
+  if (m == 0) return KNN_OK;
+  if (!idx || !out) {
+    set_error("cloud rows: null pointer argument");
+    return KNN_EINVAL;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  Arena ar(s);
+  std::vector<int32_t> off(2 * (size_t)(ncloud + 1));
+  for (int c = 0; c <= ncloud; c++) {
+    off[c] = (int32_t)q_offsets[c];
+    off[ncloud + 1 + c] = (int32_t)r_offsets[c];
+  }
+  int32_t *dev;
+  KNN_TRY(ar.alloc(&dev, off.size()));
+  KNN_TRY(upload_words(off.data(), off.size(), dev, s));
+  const int64_t blocks = std::min<int64_t>((m * k + 255) / 256, 148 * 16);
+  cloud_rows_kernel<<<(unsigned)blocks, 256, 0, s>>>(idx, m, k, dev, dev + ncloud + 1, ncloud, out);
+  KNN_LAUNCH_CHECK();
+  return KNN_OK;
+}

@@ -1148,7 +1148,9 @@ static int launch_scan_n(const ScanArgs &a, int num_sms, cudaStream_t s) {
 // surface clouds, k = 16: search 59.4 -> 20.4 ms.  64-bit keys in the merges
 // instead of distance words: 32 ms; whole clusters by their distance band
 // instead of blocks by their boxes: 22.4 ms; candidates stored by predicated
-// instructions instead of a branch: 22.4 ms.
+// instructions instead of a branch: 22.4 ms.  At k = 8 five blocks per SM
+// (96 registers) instead of six, which spilled: 64 pairs of clouds, loss and
+// gradients 3.70 -> 3.41 ms.
 //
 // FP64 boundary: the threshold is band_hi of the k-th key, so every point
 // inside the final k-th's FP32 band is evaluated and admitted; one that a merge
@@ -1317,7 +1319,7 @@ struct LaneTopK {
 __host__ __device__ constexpr int group_warps(int K) { return K > 16 ? 2 : 4; }
 
 template <int DP4, bool IDXROW, int K>
-__global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 8 ? 5 : 6))
+__global__ void __launch_bounds__(group_warps(K) * 32, K > 16 ? 8 : (K > 1 ? 5 : 6))
     group_scan_kernel(const ScanArgs a) {
   using TK = LaneTopK<K>;
   constexpr int kGroupWarps = group_warps(K);
