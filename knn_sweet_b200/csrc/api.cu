@@ -477,7 +477,9 @@ int build_query_side(const RefSide &R, bool share, const float *q, int64_t m, in
     KNN_TRY(build_clusters(ar, ar, Q->Qp, m, d, dp4s, Rq, o.seed, o.rep_trials, o.lloyd_iters,
                            use_tc, dev_err, s, &Q->qset));
     Q->order = Q->qset.perm;
-    if (narrow_rows(R.tmpl)) {
+    // (a warp per query does not mind the order: only enough queries for the
+    // group scan are worth a launch)
+    if (narrow_rows(R.tmpl) && m >= 8192) {
       int32_t *order;
       KNN_TRY(ar.alloc(&order, (size_t)m));
       KNN_TRY(launch_block_order(Q->Qp, dp4s, d, Q->qset.reps, Q->qset.skeys, Q->qset.off,
