@@ -68,7 +68,7 @@ namespace knnsweet {
 // starts and ends): kept out of registers, which the scan loop needs.
 enum {
   kStatPushed = 0, kStatMerges, kStatVisited, kStatPruned, kStatChecked,
-  kSideSlot, kSideQuery, kSideCluster, kSideDq, kStatWords
+  kSideSlot, kSideQuery, kSideCluster, kSideDq, kSideKept, kStatWords
 };
 constexpr int kStatKeys = (kStatWords + 1) / 2;  // 64-bit words they take
 
@@ -92,7 +92,17 @@ struct TopKBase {
     if (lane == 0) stat()[which] += v;
   }
 
+  // statistics: candidates pushed since the last compaction left `kept`
+  __device__ __forceinline__ void settle(int now, int kept, int lane) const {
+    if (lane == 0) {
+      unsigned *s = stat();
+      s[kStatPushed] += (unsigned)(now - (int)s[kSideKept]);
+      s[kSideKept] = (unsigned)kept;
+    }
+  }
+
   __device__ __forceinline__ void reset_threshold(float th0, int lane) {
+    if (lane == 0) stat()[kSideKept] = 0;
     nbuf = 0;
     nlist = 0;
     theta = th0;
@@ -122,7 +132,7 @@ template <int E>
 struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3> {
   using B = TopKBase<64 * E + 2, 64 * E + 3>;
   using B::buf, B::nbuf, B::nlist, B::k, B::count, B::note_lost, B::set_band_threshold,
-      B::reset_threshold;
+      B::reset_threshold, B::settle;
   static constexpr int L = 32 * E;
   static constexpr int kCap = L;  // candidate buffer capacity
   // append buffer (L keys), L doubles for the FP64 band, 2 pivot words,
@@ -168,6 +178,7 @@ struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3> {
     note_lost(lost, lane);
     reg_bitonic_merge<E>(v, lane);
     nlist = min(k, nlist + nbuf);
+    settle(nbuf, 0, lane);
     count(kStatMerges, 1, lane);
     nbuf = 0;
     if (nlist == k) {
@@ -241,7 +252,7 @@ template <int LL>
 struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
   using B = TopKBase<2 * LL + 128, 2 * LL + 129>;
   using B::buf, B::nbuf, B::nlist, B::k, B::count, B::note_lost, B::set_band_threshold,
-      B::reset_threshold;
+      B::reset_threshold, B::settle;
   static constexpr int L = LL;          // final sort length (pow2 >= k)
   static constexpr int kCap = 2 * LL;   // candidate capacity
   // keys, 256-word histogram, lostmin, statistics
@@ -286,6 +297,7 @@ struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
     }
     __syncwarp();
     note_lost(lost, lane);
+    settle(nbuf, w, lane);
     nbuf = w;  // == k
     nlist = k;
     count(kStatMerges, 1, lane);
@@ -321,6 +333,7 @@ struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
       w += __popc(bm);
     }
     __syncwarp();
+    settle(nbuf, w, lane);
     nbuf = w;
     if (w > kCap - 32) {
       flush(lane, d);
@@ -334,7 +347,7 @@ struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
   // The candidates are in buf[0..nbuf) already.
   __device__ __forceinline__ int expose(int) { return nbuf; }
   // End of the query: nothing to do before sorted().
-  __device__ __forceinline__ void finish(int, int) {}
+  __device__ __forceinline__ void finish(int lane, int) { settle(nbuf, nbuf, lane); }
 
   // The candidates, sorted, into buf[0..n); returns n.  Up to L keys are
   // sorted as they are; beyond that a band-inclusive compaction first, and
@@ -391,8 +404,7 @@ __device__ __forceinline__ void topk_offer(TK &tk, bool pass, float v, int32_t i
     cnt = __popc(b);
   }
   if (pass) tk.buf[tk.nbuf + __popc(b & ((1u << lane) - 1))] = make_key(v, idx);
-  tk.nbuf += cnt;
-  tk.count(kStatPushed, cnt, lane);
+  tk.nbuf += cnt;  // (counted by settle, not here: every step comes this way)
 }
 
 // Whether every FP32 squared distance of the join is exact (both sides hold
@@ -857,9 +869,12 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       }
       // visit this chunk's surviving clusters, nearest d(q, Rs) first
       unsigned amask = __ballot_sync(kFull, alive);
-      tk.count(kStatPruned, (unsigned)(batch - __popc(amask)), lane);
-      if (amask == 0) continue;  // warp-uniform: nothing to visit in this batch
+      if (amask == 0) {  // warp-uniform: nothing to visit in this batch
+        tk.count(kStatPruned, (unsigned)batch, lane);
+        continue;
+      }
       const int nalive = __popc(amask);
+      int visits = 0;  // counted once per batch
       float dkey = alive ? D : __int_as_float(0x7f800000);
       // Visit order: nearest d(q, Rs) first.  Narrow rows sort the batch once
       // (bitonic network over the 32 lanes, ties to the lower lane: less work
@@ -923,7 +938,6 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         float th = tk.theta;
         float slack = tol * (2.0f * Dc + 2.0f * th);
         if (Dc - cmax_c > th + slack || Dc + th + slack < cmin_c) {
-          tk.count(kStatPruned, 1, lane);
           continue;
         }
         if (kWideRows && steps > kFarSteps && a.far_slot && !split) {
@@ -937,7 +951,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           }
           steps = -(1 << 30);  // no room: the warp carries on
         }
-        tk.count(kStatVisited, 1, lane);
+        visits++;
         const int start = __shfl_sync(kFull, cst, src);
         const int n_c = __shfl_sync(kFull, cnn, src);
         if constexpr (kBlocks) {
@@ -1018,6 +1032,11 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
           step(start, p, p < n_c && ds >= lo_v && ds <= hi_v);
           if (__shfl_sync(kFull, ds > hi_v, 31)) break;
         }
+      }
+      if (lane == 0) {
+        unsigned *st = tk.stat();
+        st[kStatVisited] += (unsigned)visits;
+        st[kStatPruned] += (unsigned)(batch - visits);
       }
       if (kWideRows && far) break;
     }
