@@ -587,6 +587,8 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
     t.work = ctr + kCtrTileWork;
     t.fb_slots = fb_slots;
     t.fb_count = fb_count;
+    KNN_TRY(ar.alloc(&t.far_tiles, 1));
+    KNN_CUDA_TRY(cudaMemsetAsync(t.far_tiles, 0, sizeof(unsigned), s));
     t.err = reinterpret_cast<int *>(ctr + kCtrErr);
     t.counters = ctr + kCtrTile;
     KNN_TRY(launch_tile_search(t, grid, smem, s));

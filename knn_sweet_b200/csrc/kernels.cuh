@@ -206,6 +206,7 @@ struct TileArgs {
   unsigned long long *work;  // tile counter, zeroed
   int32_t *fb_slots;         // slots left to the FP32 scan
   unsigned *fb_count;
+  unsigned *far_tiles;       // tiles left to it for their reach, zeroed
   int *err;                  // set when a bounded wait gives up
   unsigned long long *counters;  // [tensor pairs, refined, fp64 rechecks, fallbacks]
 };

@@ -666,7 +666,11 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
           s_rlo[tid] = lo;
           s_roff[tid] = before + incl - len;
         }
-        if (tid == kTM - 1) s_wmax[1] = (uint32_t)(before + incl);
+        if (tid == kTM - 1) {
+          const bool far = before + incl > KNN_TILE_MAX_RUN &&
+                           atomicAdd(a.far_tiles, 1u) <= gridDim.x / 8;
+          s_wmax[1] = far ? 0xffffffffu : (uint32_t)(before + incl);
+        }
       }
       __syncthreads();
       const int total = (int)s_wmax[1];
@@ -683,8 +687,12 @@ __global__ void __launch_bounds__(NT, NT == kTM ? 4 : 2)
       // a tile whose queries reach too far for this form (a cluster that spans
       // distant groups of points: loose bounds, every member a candidate) goes
       // to the FP32 scan as a whole, before it streams them: one such tile took
-      // as long as all others together
-      if (total > KNN_TILE_MAX_RUN) {
+      // as long as all others together.  Only an eighth of the resident CTAs'
+      // number of tiles: with more of them no tile is alone at the end, and a
+      // tile's stream then costs less than 128 queries of the FP32 scan
+      // (N = 359,466, M = 59,911, d = 31, k = 50, no refinement, where nearly every
+      // tile reaches that far: all of them handed over 26 ms, 13 with this)
+      if (total < 0) {
         ovf = true;
         break;
       }

@@ -68,6 +68,18 @@ def test_tile_that_reaches_too_far(cuda_device, oracle):
     assert st.refine_fallbacks > 0
 
 
+def test_most_tiles_reach_too_far(cuda_device, oracle):
+    # more such tiles than may be handed back: the others are streamed
+    rng = np.random.default_rng(10)
+    r = rng.standard_normal((40_000, 16)).astype(np.float32)
+    q = rng.standard_normal((6000, 16)).astype(np.float32)
+    idx, dist, st = knnjoin(q, r, 20, qreps=40, sreps=3, precision="bf16_refine", stats=True)
+    rows = rng.permutation(6000)[:400]
+    oi, od = oracle.bruteforce_f64(q[rows], r, 20)
+    assert_matches(idx[rows], dist[rows], oi, od)
+    assert 0 < st.refine_fallbacks < 6000
+
+
 @pytest.mark.parametrize("m", [1500, 5000])
 def test_queries_left_to_a_block(cuda_device, oracle, m):
     # four clusters of 15,000 rows: every query passes the step limit of a warp
