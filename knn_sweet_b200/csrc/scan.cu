@@ -1974,8 +1974,15 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
   // k = 16: 10,000 points 139 / 68, 32,000 231 / 193, 50,000 246 / 301,
   // 100,000 395 / 635, 10^6 2220 / 8271; k = 1: 10,000 61 / 51, 16,000 70 / 74,
   // 32,000 84 / 137; k = 32: 50,000 301 / 336.
+  // The box of 32 queries grows with the dimension and reaches blocks that none
+  // of them needs, so more than 4 dimensions take it for small k only.  Whole
+  // self-joins of Gaussian mixtures in ms, group / warp: d = 4, k = 16, 140,170
+  // points 1.7 / 1.9; d = 5, k = 16 3.8 / 3.5; d = 6, k = 16 7.5 / 5.5, k = 8,
+  // 245,000 points 9.4 / 9.4 (another set 5.1 / 5.9); d = 8, k = 8 26.5 / 22.1
+  // (9.1 / 10.4); k = 1, 60,000 points, d = 6 0.77 / 1.14, d = 8 1.2 / 1.7.
   const int64_t fill = (int64_t)num_sms * 32 * (a.k == 1 ? 3 : 8);
-  if (a.k <= 32 && a.m >= fill && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
+  const int group_k = a.d <= 4 ? 32 : (a.d <= 6 ? 8 : 4);
+  if (a.k <= group_k && a.m >= fill && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
       return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)
                           : launch_group_scan<1, false>(a, num_sms, s);

@@ -33,6 +33,14 @@ def test_group_scan_float_rows(cuda_device, oracle, d, k):
     _check(oracle, q, r, k)
 
 
+@pytest.mark.parametrize("d,k", [(5, 8), (6, 8), (6, 9), (7, 4), (7, 5), (8, 4), (8, 5)])
+def test_group_scan_limit_of_k(cuda_device, oracle, d, k):
+    rng = np.random.default_rng(10 * d + k)
+    r = rng.standard_normal((2049, d)).astype(np.float32)
+    q = rng.standard_normal((MANY, d)).astype(np.float32)
+    _check(oracle, q, r, k)
+
+
 @pytest.mark.parametrize("n", [1, 3, 31, 32, 33, 1023, 1024, 1025])
 def test_group_scan_reference_sizes(cuda_device, oracle, n):
     rng = np.random.default_rng(n)
