@@ -1073,7 +1073,8 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       tk.count(kStatChecked, emit_query(tk, a, e_slot, e_q, e_qc, lane), lane);
     }
     __syncwarp();
-    if (a.counters) {
+    // (a query left to a block starts again there and is counted there)
+    if (a.counters && !far) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) evals += __shfl_xor_sync(kFull, evals, o);
       if (lane == 0) {

@@ -92,3 +92,17 @@ def test_queries_left_to_a_block(cuda_device, oracle, m):
     oi, od = oracle.bruteforce_f64(q[rows], r, 40)
     assert_matches(idx[rows], dist[rows], oi, od)
     assert (idx >= 0).all()
+
+
+@pytest.mark.parametrize("m", [3000, 5000])
+def test_statistics_of_queries_left_to_a_block(cuda_device, m):
+    # no cluster is out of reach and every query passes the step limit: each of
+    # its distances and list entries counts once
+    rng = np.random.default_rng(m)
+    n, reps = 60_000, 4
+    r = rng.standard_normal((n, 16)).astype(np.float32)
+    q = (3 * rng.standard_normal((m, 16))).astype(np.float32)
+    st = knnjoin(q, r, 40, sreps=reps, qreps=8, stats=True)[2]
+    assert 0 < st.dist_evals <= st.pairs_total == m * n
+    assert st.pairs_pruned == st.pairs_total - st.dist_evals
+    assert st.clusters_visited + st.clusters_pruned <= m * reps
