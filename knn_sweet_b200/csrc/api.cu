@@ -695,6 +695,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
       ScanArgs ac = a;
       ac.slot_list = cslots + r0;
       ac.slot_count = reinterpret_cast<const unsigned *>(ccount + c);
+      ac.list_full = true;
       ac.m = counts[c];
       ac.work_counter = cwork + c;
       KNN_TRY(launch_scan(ac, num_sms, s));
@@ -716,6 +717,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
       KNN_TRY(launch_slot_order(Q.slot_cl, Q.qset.off, cstart, m, order, count, s));
       a.slot_list = order;
       a.slot_count = count;
+      a.list_full = true;
     }
     KNN_TRY(launch_scan(a, num_sms, s));
   }

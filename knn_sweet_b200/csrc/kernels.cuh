@@ -60,6 +60,7 @@ struct ScanArgs {
                                // index of query cluster qc (null: 0)
   const int32_t *slot_list;    // optional: scan only these slots ...
   const unsigned *slot_count;  // ... *slot_count of them (device count);
+  bool list_full;              // ... which is m
   int split_max;               // a block per query up to this many (launch_scan)
   int32_t *far_slot;           // optional (wide rows): room for kFarQueries slots,
   unsigned *far_count;         // and their number: queries the scan gave up on,

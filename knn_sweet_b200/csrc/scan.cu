@@ -112,9 +112,9 @@ struct TopKBase {
   }
   // threshold once the k-th squared distance is T: the FP32 band above it
   __device__ __forceinline__ void set_band_threshold(float T, int d) {
-    const float W = band_hi(T, d);
-    thr_d2 = W;
-    theta = sqrtf(W);
+    // (a threshold from the block's other warps may lie lower)
+    thr_d2 = fminf(thr_d2, band_hi(T, d));
+    theta = sqrtf(thr_d2);
   }
   // a dropped key's distance word (NaN from an empty key is ignored)
   __device__ __forceinline__ void note_lost(uint32_t d2bits, int lane) {
@@ -198,6 +198,13 @@ struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3> {
     }
   }
 
+  // Lane l: a d^2 word that at least l + 1 candidates do not exceed (all ones:
+  // fewer).
+  __device__ __forceinline__ uint32_t nearest(int lane, int d) {
+    static_assert(E == 1, "one key per lane");
+    flush(lane, d);
+    return (uint32_t)(v[0] >> 32);
+  }
   // The candidates into buf[0..n) for another warp; returns n.
   __device__ __forceinline__ int expose(int lane) { return sorted(lane, 0); }
   // The candidates, sorted, into buf[0..n); returns n.
@@ -344,6 +351,22 @@ struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
     set_band_threshold(__uint_as_float(T), d);
   }
 
+  // Lane l: a d^2 word that at least l + 1 candidates do not exceed (all ones:
+  // fewer), the l-th of the 32 lanes' minima.
+  __device__ __forceinline__ uint32_t nearest(int lane, int) {
+    __syncwarp();
+    uint32_t x = 0xffffffffu;
+    for (int i = lane; i < nbuf; i += 32) x = min(x, (uint32_t)(buf[i] >> 32));
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        const uint32_t o = __shfl_xor_sync(kFull, x, stride);
+        x = ((lane & stride) == 0) == ((lane & size) == 0) ? min(x, o) : max(x, o);
+      }
+    }
+    return x;
+  }
   // The candidates are in buf[0..nbuf) already.
   __device__ __forceinline__ int expose(int) { return nbuf; }
   // End of the query: nothing to do before sorted().
@@ -691,15 +714,25 @@ constexpr int scan_min_blocks() {
   return ((DP4 == 0 || DP4 >= 4) ? KNN_TARGET_WARPS_WIDE : KNN_TARGET_WARPS) / WARPS;
 }
 
-// Steps of 32 members after which a warp leaves its query of wide rows to a
-// whole block (a launch behind the scan's): a few queries between distant
-// groups of points reach a hundred times the members of the others, and the
-// scan took as long as the longest (N = 10^6, d = 32, k = 32, six data sets:
-// 2.9 to 5.5 ms, 2.9 to 3.3 with this).
+// A query of wide rows may be left to a whole block (a launch behind the
+// scan's): a few queries between distant groups of points reach a hundred
+// times the members of the others, and the scan took as long as the longest
+// (N = 10^6, d = 32, k = 32, six data sets: 2.9 to 5.5 ms, 2.9 to 3.3 with
+// this).  The block starts it again, so a query goes only after kFarSteps steps
+// of 32 members, when two thirds of the warps have no query left to take, and
+// with most of a list that can be dealt out to warps before it.  Any query of
+// that many steps, idle warps or not: 100,000 rows, d = 16, four clusters,
+// 2,300 queries 8.2 ms; warps that keep them 2.5; 200,003 rows, d = 64, 3,000
+// queries: none given up 20.0, with a third of the warps busy 15.4.
 constexpr int kFarSteps = 512;
+// Entries from which on a list is dealt out to a block's warps; of a shorter one
+// they take parts of every cluster.  100,000 rows, d = 32 in 500 distant groups, 16
+// clusters, 500 queries, k = 50: dealt out 1,017 us (a warp per query 605), in parts
+// 500; one Gaussian, d = 16, 16 clusters: 992 and 1,278 (2,097).
+constexpr int kShareLists = 32;
 
 // ONE: the reference set is a single cluster of narrow rows (small joins).
-template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
+template <int DP4, bool IDXROW, int L, int WARPS, bool ONE, bool SPLIT>
 __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     scan_kernel(const ScanArgs a) {
   using TK = TopKFor<L>;
@@ -725,23 +758,30 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
   if (lane < kStatWords) tk.stat()[lane] = 0;
   __syncthreads();
 
-  // Few queries of wide rows (at most split_max): the block's warps share one
-  // query, each takes every WARPS-th cluster of its list, all tighten one
-  // threshold (s_thr, distance bits), and warp 0 merges their candidates
-  __shared__ unsigned s_thr;
+  // SPLIT: the block's warps share one query, all tighten one threshold (s_thr,
+  // distance bits), and warp 0 merges their candidates.  A list of many
+  // clusters is dealt out, each warp takes every WARPS-th cluster; of a list of
+  // few (kShareLists) every warp walks all clusters, but takes every
+  // WARPS-th block of 32 members of each.  Then one warp's k-th is far above the
+  // block's: s_part[w][j] is a d^2 word that j + 1 of warp w's candidates do not
+  // exceed, and the k-th smallest of all these words bounds the k-th distance
+  // (words only fall, so a word read late is still true)
+  __shared__ unsigned s_thr, s_part[SPLIT ? WARPS : 1][32];
   __shared__ long long s_slot;
   // (more may have been counted than there was room for in the far list)
-  const int64_t listed =
+  const int64_t listed_all =
       a.slot_list ? min((int64_t)*a.slot_count, a.m) : a.m;
-  const bool split = kWideRows && listed <= (int64_t)a.split_max;
+  // (of a list whose length only the device knows, one of two launches returns)
+  if (kWideRows && (SPLIT ? listed_all > a.split_max : listed_all <= a.split_max)) return;
   for (;;) {
     long long slot = 0;
-    if (split) {
+    if constexpr (SPLIT) {
       __syncthreads();
       if (threadIdx.x == 0) {
         s_slot = (long long)atomicAdd(a.work_counter, 1ull);
         s_thr = 0x7f800000u;
       }
+      s_part[w][lane] = 0xffffffffu;
       __syncthreads();
       slot = s_slot;
     } else {
@@ -749,7 +789,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       slot = __shfl_sync(kFull, slot, 0);
     }
     if (a.slot_list) {
-      if (slot >= listed) break;
+      if (slot >= listed_all) break;
       slot = a.slot_list[slot];
     } else if (slot >= a.m) {
       break;
@@ -782,7 +822,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     int steps = 0;      // (wide rows: how far the query has come ...
     bool far = false;   // ... and whether it is left to a whole block)
     auto step = [&](int start, int p, bool in) {
-      if constexpr (kWideRows) steps++;
+      if constexpr (kWideRows && !SPLIT) steps++;
       const unsigned gp = (unsigned)(start + p);
       float v = 0.0f;
       int32_t idx = 0;
@@ -812,8 +852,40 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
 
     const int nr = a.rlen[qc];
     const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
-    // (split: entry j of the list is warp j % WARPS's)
-    const int every = split ? WARPS : 1, first = split ? w : 0;
+    const bool share = SPLIT && nr < kShareLists;
+    const int every = SPLIT && !share ? WARPS : 1, first = SPLIT && !share ? w : 0;
+    const bool tally = !share || w == 0;  // list entries count once
+    // the smallest threshold that some warp, or all of them together, know
+    auto exchange = [&]() {
+      if constexpr (SPLIT) {
+        unsigned t = __float_as_uint(tk.thr_d2);
+        if (share && a.k <= 32 * WARPS) {
+          volatile unsigned(*part)[32] = s_part;
+          part[w][lane] = min((unsigned)part[w][lane], tk.nearest(lane, a.d));
+          __syncwarp();
+          unsigned x[WARPS];
+#pragma unroll
+          for (int o = 0; o < WARPS; o++) x[o] = part[o][lane];
+          // the k-th smallest, its last 10 bits rounded up
+          unsigned kth = 0;
+          for (int bit = 30; bit >= 10; bit--) {
+            const unsigned upto = kth | ((1u << bit) - 1);
+            int cnt = 0;
+#pragma unroll
+            for (int o = 0; o < WARPS; o++) cnt += x[o] <= upto;
+            if ((int)__reduce_add_sync(kFull, (unsigned)cnt) < a.k) kth |= 1u << bit;
+          }
+          kth |= 1023u;
+          if (kth < 0x7f800000u) t = min(t, __float_as_uint(band_hi(__uint_as_float(kth), a.d)));
+        }
+        if (lane == 0) t = min(atomicMin(&s_thr, t), t);
+        const float tv = __uint_as_float(__shfl_sync(kFull, t, 0));
+        if (tv < tk.thr_d2) {
+          tk.thr_d2 = tv;
+          tk.theta = sqrtf(tv);
+        }
+      }
+    };
     for (int base = 0; base < nr; base += 32 * every) {
 #if KNN_CHUNK_EXIT
       // the rest of the list is prunable when even its nearest cluster
@@ -828,7 +900,8 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const float2 cb = a.clb[(size_t)sw[kSideCluster] * a.clb_stride + (base >> 5)];
         const float dqv = __uint_as_float(sw[kSideDq]), th = tk.theta;
         if (cb.x - dqv - cb.y > th + 2.0f * tol * (cb.x + dqv + cb.y + th)) {
-          tk.count(kStatPruned, (unsigned)(max(nr - base - first, 0) + every - 1) / every, lane);
+          if (tally)
+            tk.count(kStatPruned, (unsigned)(max(nr - base - first, 0) + every - 1) / every, lane);
           break;
         }
       }
@@ -844,7 +917,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         if (listed)
           listed = !(a.rlb[(size_t)(rl - a.rlist) + j] - dqv > th + 2.0f * tol * (dqv + th));
         if (!__any_sync(kFull, listed)) {
-          tk.count(kStatPruned, (unsigned)batch, lane);
+          if (tally) tk.count(kStatPruned, (unsigned)batch, lane);
           continue;
         }
       }
@@ -870,7 +943,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       // visit this chunk's surviving clusters, nearest d(q, Rs) first
       unsigned amask = __ballot_sync(kFull, alive);
       if (amask == 0) {  // warp-uniform: nothing to visit in this batch
-        tk.count(kStatPruned, (unsigned)batch, lane);
+        if (tally) tk.count(kStatPruned, (unsigned)batch, lane);
         continue;
       }
       const int nalive = __popc(amask);
@@ -925,31 +998,31 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const float Dc = __shfl_sync(kFull, D, src);
         const float cmax_c = __shfl_sync(kFull, cmx, src);
         const float cmin_c = __shfl_sync(kFull, cmn, src);
-        if (split) {
-          unsigned t = 0;
-          if (lane == 0) t = min(atomicMin(&s_thr, __float_as_uint(tk.thr_d2)),
-                                 __float_as_uint(tk.thr_d2));
-          const float tv = __uint_as_float(__shfl_sync(kFull, t, 0));
-          if (tv < tk.thr_d2) {
-            tk.thr_d2 = tv;
-            tk.theta = sqrtf(tv);
-          }
-        }
+        exchange();
         float th = tk.theta;
         float slack = tol * (2.0f * Dc + 2.0f * th);
         if (Dc - cmax_c > th + slack || Dc + th + slack < cmin_c) {
           continue;
         }
-        if (kWideRows && steps > kFarSteps && a.far_slot && !split) {
-          unsigned at = 0;
-          if (lane == 0) at = atomicAdd(a.far_count, 1u);
+        if (kWideRows && !SPLIT && steps > kFarSteps && a.far_slot && nr >= kShareLists &&
+            2 * (base + rank) < nr) {
+          // (every pull from the work counter past the last query is a warp that
+          // has gone)
+          unsigned at = kFarQueries;
+          if (lane == 0) {
+            const unsigned long long warps = (unsigned long long)gridDim.x * WARPS;
+            const unsigned long long taken =
+                *reinterpret_cast<volatile unsigned long long *>(a.work_counter);
+            if (taken >= (unsigned long long)listed_all + warps - warps / 3)
+              at = atomicAdd(a.far_count, 1u);
+          }
           at = __shfl_sync(kFull, at, 0);
           if (at < kFarQueries) {
             if (lane == 0) a.far_slot[at] = (int32_t)slot;
             far = true;
             break;
           }
-          steps = -(1 << 30);  // no room: the warp carries on
+          steps = kFarSteps - 64;  // looks again after 64 steps
         }
         visits++;
         const int start = __shfl_sync(kFull, cst, src);
@@ -1020,20 +1093,33 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
         const float lo_edge = Dc - th - slack;
         const int lo = lo_edge <= cmin_c ? 0 : warp_lower_bound_coarse(a.sdist + start, n_c, lo_edge, lane);
         const float inf = __int_as_float(0x7f800000);
-        float dsv = lo + lane < n_c ? a.sdist[start + lo + lane] : inf;
-        for (int p0 = lo; p0 < n_c; p0 += 32) {
-          th = tk.theta;
-          slack = tol * (2.0f * Dc + 2.0f * th);
-          const float hi_v = Dc + th + slack, lo_v = Dc - th - slack;
-          const int p = p0 + lane;
-          const float ds = dsv;
-          // the next step's band distances come while this one's rows do
-          dsv = p + 32 < n_c ? a.sdist[start + p + 32] : inf;
-          step(start, p, p < n_c && ds >= lo_v && ds <= hi_v);
-          if (__shfl_sync(kFull, ds > hi_v, 31)) break;
+        auto walk = [&](int from, auto stride, auto every_step) {
+          float dsv = from + lane < n_c ? a.sdist[start + from + lane] : inf;
+          for (int p0 = from; p0 < n_c; p0 += stride.value) {
+            every_step(p0);
+            th = tk.theta;
+            slack = tol * (2.0f * Dc + 2.0f * th);
+            const float hi_v = Dc + th + slack, lo_v = Dc - th - slack;
+            const int p = p0 + lane;
+            const float ds = dsv;
+            // the next step's band distances come while this one's rows do
+            dsv = p + stride.value < n_c ? a.sdist[start + p + stride.value] : inf;
+            step(start, p, p < n_c && ds >= lo_v && ds <= hi_v);
+            if (__shfl_sync(kFull, ds > hi_v, 31)) break;
+          }
+        };
+        if (SPLIT && share) {
+          // blocks at multiples of 32, wherever this warp's edge lies
+          const int b = lo >> 5;
+          walk(32 * (b + ((w - b) & (WARPS - 1))), std::integral_constant<int, 32 * WARPS>(),
+               [&](int p0) {
+                 if (((p0 / (32 * WARPS)) & 3) == 3) exchange();
+               });
+        } else {
+          walk(lo, std::integral_constant<int, 32>(), [](int) {});
         }
       }
-      if (lane == 0) {
+      if (lane == 0 && tally) {
         unsigned *st = tk.stat();
         st[kStatVisited] += (unsigned)visits;
         st[kStatPruned] += (unsigned)(batch - visits);
@@ -1041,7 +1127,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       if (kWideRows && far) break;
     }
     tk.finish(lane, a.d);
-    if (split) {
+    if constexpr (SPLIT) {
       // the other warps' candidates, into warp 0's
       if (w > 0) {
         const int cnt = tk.expose(lane);
@@ -1065,7 +1151,7 @@ __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
       }
     }
     __syncwarp();
-    if ((!split || w == 0) && !far) {
+    if ((!SPLIT || w == 0) && !far) {
       const unsigned *sw = tk.stat();
       const int32_t e_slot = (int32_t)sw[kSideSlot];
       const int64_t e_q = (int64_t)sw[kSideQuery];
@@ -1108,23 +1194,39 @@ constexpr int kSplitWaves = 4;
 template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
   using TK = TopKFor<L>;
+  constexpr bool kWideRows = DP4 == 0 || DP4 >= 4;
   const size_t smem = (size_t)WARPS * TK::kSmemKeys * sizeof(uint64_t) +
                       (DP4 > 0 ? 0 : (size_t)WARPS * a.dp4 * sizeof(float4));
-  auto kern = scan_kernel<DP4, IDXROW, L, WARPS, ONE>;
-  if (smem > 48 * 1024)
-    KNN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-  int per_sm = 0;
-  KNN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
-  if (per_sm < 1) per_sm = 1;
-  int64_t grid = (int64_t)num_sms * per_sm;
+  auto resident = [&](auto kern, int64_t *blocks) -> int {
+    if (smem > 48 * 1024)
+      KNN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem));
+    int per_sm = 0;
+    KNN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
+    *blocks = (int64_t)num_sms * std::max(per_sm, 1);
+    return KNN_OK;
+  };
   ScanArgs b = a;
-  // (the queries left by a first launch are always split)
-  b.split_max = a.split_max > 0 ? a.split_max : (int)(kSplitWaves * grid);
-  const int64_t want = a.m <= b.split_max ? a.m : (a.m + WARPS - 1) / WARPS;
-  if (grid > want) grid = want;
-  if (grid < 1) grid = 1;
-  kern<<<(int)grid, WARPS * 32, smem, s>>>(b);
+  if constexpr (kWideRows) {
+    auto kern = scan_kernel<DP4, IDXROW, L, WARPS, ONE, true>;
+    int64_t grid = 0;
+    const int rc = resident(kern, &grid);
+    if (rc != KNN_OK) return rc;
+    // (the queries left by a first launch are always split)
+    if (a.split_max <= 0) b.split_max = (int)(kSplitWaves * grid);
+    // (a list may turn out shorter than its room)
+    const bool known = !a.slot_list || a.list_full;
+    if (a.m <= b.split_max || !known) {
+      kern<<<(int)std::min(grid, a.m), WARPS * 32, smem, s>>>(b);
+      KNN_LAUNCH_CHECK();
+    }
+    if (a.m <= b.split_max) return KNN_OK;
+  }
+  auto kern = scan_kernel<DP4, IDXROW, L, WARPS, ONE, false>;
+  int64_t grid = 0;
+  const int rc = resident(kern, &grid);
+  if (rc != KNN_OK) return rc;
+  kern<<<(int)std::min<int64_t>(grid, (a.m + WARPS - 1) / WARPS), WARPS * 32, smem, s>>>(b);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }

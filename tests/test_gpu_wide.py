@@ -106,3 +106,46 @@ def test_statistics_of_queries_left_to_a_block(cuda_device, m):
     assert 0 < st.dist_evals <= st.pairs_total == m * n
     assert st.pairs_pruned == st.pairs_total - st.dist_evals
     assert st.clusters_visited + st.clusters_pruned <= m * reps
+
+
+@pytest.mark.parametrize("k", [1, 8, 24, 25, 64, 200, 256, 257, 700])
+@pytest.mark.parametrize("sreps", [1, 2, 31, 33])
+def test_few_queries_few_clusters(cuda_device, oracle, k, sreps):
+    # a block per query, its warps sharing every cluster (lists of fewer than 32)
+    # or dealt whole clusters; two distant groups, clusters of every remainder
+    rng = np.random.default_rng(100 * sreps + k)
+    n = 2049 + 31 * sreps
+    side = rng.integers(0, 2, (n, 1)) * 50.0
+    r = (rng.standard_normal((n, 16)) + side).astype(np.float32)
+    q = (rng.standard_normal((45, 16)) + 50.0 * rng.integers(0, 2, (45, 1))).astype(np.float32)
+    idx, dist, st = knnjoin(q, r, k, sreps=sreps, stats=True)
+    oi, od = oracle.bruteforce_f64(q, r, k)
+    assert_matches(idx, dist, oi, od)
+    assert 0 < st.dist_evals <= st.pairs_total
+    assert st.clusters_visited + st.clusters_pruned <= 45 * sreps
+
+
+@pytest.mark.parametrize("sreps", [1, 5])
+def test_few_clusters_ties(cuda_device, oracle, sreps):
+    # the k-th of the warps' shared words among crowds of equal distances
+    rng = np.random.default_rng(sreps)
+    r = rng.integers(0, 2, (3000, 10)).astype(np.float32)
+    q = rng.integers(0, 2, (20, 10)).astype(np.float32)
+    for k in (2, 24, 60):
+        idx, dist = knnjoin(q, r, k, sreps=sreps)
+        oi, od = oracle.bruteforce_f64(q, r, k)
+        assert_matches(idx, dist, oi, od, exact=True)
+
+
+@pytest.mark.parametrize("k", [10, 40])
+def test_long_lists_left_to_a_block(cuda_device, oracle, k):
+    # no cluster out of reach, 100 of them: the last queries go to a block each
+    rng = np.random.default_rng(k)
+    r = rng.standard_normal((60_000, 16)).astype(np.float32)
+    q = (2 * rng.standard_normal((6000, 16))).astype(np.float32)
+    idx, dist, st = knnjoin(q, r, k, sreps=100, qreps=8, stats=True)
+    rows = rng.permutation(6000)[:200]
+    oi, od = oracle.bruteforce_f64(q[rows], r, k)
+    assert_matches(idx[rows], dist[rows], oi, od)
+    assert (idx >= 0).all()
+    assert 0 < st.dist_evals <= st.pairs_total
