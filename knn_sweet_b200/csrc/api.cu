@@ -627,6 +627,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   a.clb_stride = (Rs + 31) / 32;
   a.Rs = Rs;
   a.n_ref = R.n;
+  a.m_near = m;
   a.rrows = R.Rp;
   a.inexact_r = R.inexact;
   a.inexact_q = Q.inexact;
@@ -696,7 +697,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
       ac.slot_list = cslots + r0;
       ac.slot_count = reinterpret_cast<const unsigned *>(ccount + c);
       ac.list_full = true;
-      ac.m = counts[c];
+      ac.m = ac.m_near = counts[c];  // (rows of a chunk, not neighbours in space)
       ac.work_counter = cwork + c;
       KNN_TRY(launch_scan(ac, num_sms, s));
       KNN_CUDA_TRY(cudaEventRecord((*evs)[c], s));

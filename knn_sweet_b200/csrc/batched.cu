@@ -550,6 +550,7 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       a.qc_ref_base = qc_ref_base;
       a.Rs = S.Rtot;
       a.n_ref = S.total;
+      a.m_near = m;
       a.rrows = S.rows;
       {
         int *fr = reinterpret_cast<int *>(ctr + 2 + kScanCounters);

@@ -67,8 +67,9 @@ struct ScanArgs {
                                // which get a block each afterwards
   int64_t slot_base;           // without a list: slots slot_base .. + m - 1
   int Rs;
-  int64_t n_ref;            // reference points (0: unknown); with Rs it gives
-                            // the mean cluster size the scan variant is chosen by
+  int64_t n_ref;            // reference points; with Rs the mean cluster size
+  int64_t m_near;           // queries that neighbouring slots are drawn from (m, or
+                            // the whole join's for a range of its slots)
   const float4 *rrows;      // n x dp4 reference rows, original order (the
                             // FP64 re-check of the k-th boundary)
   const int *inexact_r;     // device flags of the two sides, 0 when every

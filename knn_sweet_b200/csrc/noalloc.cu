@@ -369,6 +369,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   a.rlen = p.rlen;
   a.Rs = p.Rs;
   a.n_ref = n;
+  a.m_near = m;
   a.rrows = Rp;
   {
     int *fr = reinterpret_cast<int *>(p.ctr + kCtrInexactR);

@@ -2077,15 +2077,24 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
   // k = 16: 10,000 points 139 / 68, 32,000 231 / 193, 50,000 246 / 301,
   // 100,000 395 / 635, 10^6 2220 / 8271; k = 1: 10,000 61 / 51, 16,000 70 / 74,
   // 32,000 84 / 137; k = 32: 50,000 301 / 336.
-  // The box of 32 queries grows with the dimension and reaches blocks that none
-  // of them needs, so more than 4 dimensions take it for small k only.  Whole
-  // self-joins of Gaussian mixtures in ms, group / warp: d = 4, k = 16, 140,170
-  // points 1.7 / 1.9; d = 5, k = 16 3.8 / 3.5; d = 6, k = 16 7.5 / 5.5, k = 8,
-  // 245,000 points 9.4 / 9.4 (another set 5.1 / 5.9); d = 8, k = 8 26.5 / 22.1
-  // (9.1 / 10.4); k = 1, 60,000 points, d = 6 0.77 / 1.14, d = 8 1.2 / 1.7.
+  // The queries must also lie close together, against the reference points: the
+  // box of 32 distant ones reaches blocks that none of them needs, the more so
+  // the more dimensions there are.  Whole joins in us, group / warp, n reference
+  // rows by m queries, uniform points unless said otherwise: d = 3, k = 16,
+  // 150,000 by 40,000 741 / 658 (mixtures 775 to 895 / 673 to 716); d = 4, k = 16,
+  // 100,000 by 50,000 1202 / 826, 60,000 by 60,000 1073 / 850, 150,000 by 150,000
+  // 1542 / 1751; k = 4, 60,000 by themselves d = 5 1350 / 844, d = 6 2296 / 1171,
+  // d = 8 5592 / 2453 (200 mixtures 546 / 537); d = 8, k = 4, 20,000 by 200,000
+  // 4817 / 5682 (8 mixtures 1388 / 2569); d = 6, k = 4, 64 clouds of 2,000 704
+  // / 1017 (8 mixtures 380 / 618); d = 2, k = 4, 100,000 by 50,000 446 / 560.
   const int64_t fill = (int64_t)num_sms * 32 * (a.k == 1 ? 3 : 8);
   const int group_k = a.d <= 4 ? 32 : (a.d <= 6 ? 8 : 4);
-  if (a.k <= group_k && a.m >= fill && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
+  const bool tiny = a.n_ref <= 100 * (int64_t)a.Rs;  // clusters of a few blocks
+  const bool dense = a.d <= 2   ? 2 * a.m_near >= a.n_ref
+                     : a.d == 3 ? a.m_near >= a.n_ref
+                     : a.d == 4 ? tiny || a.m_near >= (a.m >= 2 * fill ? 1 : 2) * a.n_ref
+                                : tiny || a.m_near >= 4 * a.n_ref;
+  if (a.k <= group_k && a.m >= fill && dense && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
       return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)
                           : launch_group_scan<1, false>(a, num_sms, s);

@@ -271,7 +271,6 @@ int small_join(const float *q, int64_t m, const float *r, int64_t n, int d, int 
   a.rlist = &ctl->rlist;
   a.rlen = &ctl->rlen;
   a.Rs = 1;
-  a.n_ref = n;
   a.rrows = Rp;
   a.inexact_r = &ctl->inexact;
   a.inexact_q = self ? &ctl->inexact : inexact_q;

@@ -100,3 +100,15 @@ def test_small_join_self_and_missing_slots(cuda_device):
     assert idx[0].tolist() == [0, 1, 3, -1, -1, -1]
     assert dist[0, :3].tolist() == [0.0, 1.0, 3.0] and bool(torch.isinf(dist[0, 3:]).all())
     assert idx[2].tolist() == [-1] * 6  # no distance from a NaN query is a number
+
+
+@pytest.mark.parametrize("d,n,m", [(3, MANY - 1, MANY), (3, MANY + 1, MANY), (4, 40_000, 76_000),
+                                   (4, 40_000, 75_000), (6, 9000, MANY), (6, 10_000, MANY),
+                                   (8, 9600, MANY)])
+def test_group_scan_limit_of_density(cuda_device, oracle, d, n, m):
+    # enough queries for groups of 32, but as many reference rows on both sides of
+    # the limit from which they lie too far apart
+    rng = np.random.default_rng(n + d)
+    r = rng.uniform(-1, 1, (n, d)).astype(np.float32)
+    q = rng.uniform(-1, 1, (m, d)).astype(np.float32)
+    _check(oracle, q, r, 4, sample=150)
