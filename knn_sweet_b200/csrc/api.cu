@@ -615,6 +615,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   a.srows = R.srows;
   a.sdist = R.sdist;
   a.sidx = R.sidx;
+  a.dorder = R.boxes ? R.sset.perm : nullptr;
   a.soff = R.sset.off;
   a.cmin = R.cmin;
   a.cmax = R.cmax;

@@ -386,10 +386,11 @@ int cluster_side(Arena &ar, const float *pts, const int64_t *off_h, int ncloud, 
   KNN_TRY(ar.alloc(&b->off, (size_t)b->Rtot + 1));
   KNN_TRY(launch_cluster_offsets(b->skeys, b->total, b->Rtot, b->off, s));
   b->order = b->perm;
-  // (in place: nothing reads the order by distance after this)
-  if (narrow_rows(dp4))
+  if (narrow_rows(dp4)) {
+    KNN_TRY(ar.alloc(&b->order, (size_t)b->total));
     KNN_TRY(launch_block_order(b->rows, dp4, d, b->reps, b->skeys, b->off, b->perm, b->total,
                                b->order, s));
+  }
   return KNN_OK;
 }
 
@@ -538,6 +539,7 @@ int batched_impl(const float *q, const int64_t *qoff_h, const float *r, const in
       a.srows = srows;
       a.sdist = sdist;
       a.sidx = sidx;
+      a.dorder = cols ? nullptr : S.perm;
       a.soff = S.off;
       a.cmin = cmin;
       a.cmax = cmax;

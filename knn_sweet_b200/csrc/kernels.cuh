@@ -40,6 +40,8 @@ struct ScanArgs {
                             // no block is skipped)
   const float *sdist;       // n: d(s, Rs) in the same order
   const int32_t *sidx;      // n: original reference row
+  const int32_t *dorder;    // optional (narrow rows): n, the original reference
+                            // rows in the order of sdist
   const int32_t *soff;      // Rs + 1 cluster offsets
   const float *cmin, *cmax; // Rs: smallest / largest member distance
   const float *theta0;      // Rq: initial k-th bound per query cluster

@@ -308,18 +308,18 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   const float4 *Rp = nullptr, *Qp = nullptr;
   rc = cluster_side(p, p.S, r, n, p.Rs, &Rp, s);
   if (rc != KNN_OK) return rc;
-  // narrow rows: the block order in place of the order by distance, the boxes
-  // in the sort's input keys (no longer needed) where they fit: without them
-  // the scan skips whole clusters only
+  // narrow rows: the block order in the sort's input values, the boxes in its
+  // input keys (neither is needed any more) where they fit: without them the
+  // scan skips whole clusters only
   const bool narrow = narrow_rows(p.tmpl);
   float4 *boxes = nullptr;
   if (narrow) {
     if ((uint64_t)block_count(n, p.Rs) * 2 * p.dp4s * sizeof(float4) <= (uint64_t)n * 8)
       boxes = reinterpret_cast<float4 *>(p.S.keys);
-    rc = launch_block_order(Rp, p.dp4s, d, p.S.reps, p.S.skeys, p.S.off, p.S.perm, n, p.S.perm, s);
+    rc = launch_block_order(Rp, p.dp4s, d, p.S.reps, p.S.skeys, p.S.off, p.S.perm, n, p.S.vals, s);
     if (rc != KNN_OK) return rc;
   }
-  rc = launch_cluster_layout(p.S.skeys, p.S.perm, n, Rp, p.dp4s, p.idx_in_row, false, p.srows,
+  rc = launch_cluster_layout(p.S.skeys, narrow ? p.S.vals : p.S.perm, n, Rp, p.dp4s, p.idx_in_row, false, p.srows,
                              p.sdist, p.sidx, s);
   if (rc == KNN_OK && boxes)
     rc = launch_block_boxes(p.srows, p.dp4s, d, p.S.skeys, p.S.off, n, boxes, s);
@@ -331,7 +331,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   } else {
     rc = cluster_side(p, p.Q, q, m, p.Rq, &Qp, s);
     if (rc == KNN_OK && narrow)
-      rc = launch_block_order(Qp, p.dp4s, d, p.Q.reps, p.Q.skeys, p.Q.off, p.Q.perm, m, p.Q.perm,
+      rc = launch_block_order(Qp, p.dp4s, d, p.Q.reps, p.Q.skeys, p.Q.off, p.Q.perm, m, p.Q.vals,
                               s);
     if (rc != KNN_OK) return rc;
   }
@@ -343,7 +343,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   if (rc != KNN_OK) return rc;
   ScanArgs a{};
   a.qrows = Qp;
-  a.qorder = Qb.perm;
+  a.qorder = narrow ? Qb.vals : Qb.perm;
   a.qreps = Qb.reps;
   a.boxes = boxes;
   a.slot_cl = p.slot_cl;
@@ -359,6 +359,7 @@ int noalloc_join(const float *q, int64_t m, const float *r, int64_t n, int32_t d
   a.srows = p.srows;
   a.sdist = p.sdist;
   a.sidx = p.sidx;
+  a.dorder = narrow ? p.S.perm : nullptr;
   a.soff = p.S.off;
   a.cmin = p.cmin;
   a.cmax = p.cmax;

@@ -1812,6 +1812,110 @@ static int launch_group_scan(const ScanArgs &a, int num_sms, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
+// Thread per query: the self-join's nearest point (k = 1) in short clusters of
+// 5 to 8 dimensions.  The point itself or a copy of it settles a query as soon as
+// its own cluster is read, so that what is left is the walk along the cluster
+// list -- a hundred distances, each dropped by its test -- for which a query needs
+// no more than a thread, while the box of 32 queries still reaches clusters that
+// none of them does.  Members are read by their distance to the representative
+// (dorder: a row of 32 bytes is one sector wherever it lies), those of the band
+// |D - d(s,Rs)| <= theta only.  The start's bound, the FP32 keys and the FP64
+// boundary are the other scans'.  What bounds it: the latency of a thread's
+// dependent loads.  Self-joins of 30,000 uniform points, whole, group scan /
+// this: d = 5 459 / 371 us, d = 8 926 / 394; 64 clouds of 2,000, d = 8 559 / 315.
+// ---------------------------------------------------------------------------
+template <int DP4>
+__global__ void __launch_bounds__(256, 4) thread_scan_kernel(const ScanArgs a) {
+  __shared__ unsigned long long blk_ctr[4];
+  if (threadIdx.x < 4) blk_ctr[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t nslots = a.slot_list ? (int64_t)*a.slot_count : a.m;
+  const float inf = __int_as_float(0x7f800000);
+  unsigned evals = 0, visited = 0, pruned = 0, pushed = 0;
+  if (t < nslots) {
+    const int64_t slot = a.slot_list ? (int64_t)a.slot_list[t] : a.slot_base + t;
+    const int64_t q = a.qorder[slot];
+    const int qc = a.slot_cl[slot];
+    const float tol = bound_tol(a.d);
+    QueryRow<DP4, false> qr;
+    qr.load(a.qrows, q, DP4, nullptr);
+    float theta =
+        query_theta0(a, sqrtf(qr.dist2(a.qreps + (int64_t)qc * DP4, DP4)), qc, tol);
+    float thr = theta * theta;  // admits every d^2 <= theta0^2, whatever the index
+    float lost = inf;           // smallest d^2 that was admitted and is not the result
+    uint64_t best = kKeyMax;
+    const int nr = a.rlen[qc];
+    const int32_t *rl = a.rlist + (a.rl_base ? a.rl_base[qc] : (int64_t)qc * a.Rs);
+    for (int j = 0; j < nr; j++) {
+      const int c = rl[j];
+      const float D = sqrtf(qr.dist2(a.sreps + (int64_t)c * DP4, DP4));
+      float slack = tol * (2.0f * D + 2.0f * theta);
+      const float cmin = a.cmin[c];
+      if (D - a.cmax[c] > theta + slack || D + theta + slack < cmin) {
+        pruned++;
+        continue;
+      }
+      visited++;
+      const int start = a.soff[c], n_c = a.soff[c + 1] - start;
+      const float *sd = a.sdist + start;
+      // first member of the band [D - theta, D + theta] (with slack)
+      const float lo_edge = D - theta - slack;
+      int p = 0;
+      if (lo_edge > cmin) {
+        int hi = n_c;
+        while (p < hi) {
+          const int md = (p + hi) >> 1;
+          if (sd[md] < lo_edge) p = md + 1;
+          else hi = md;
+        }
+      }
+      for (; p < n_c && !(sd[p] > D + theta + slack); p++) {
+        const int32_t idx = a.dorder[start + p];
+        const float v = qr.dist2(a.rrows + (int64_t)idx * DP4, DP4);
+        evals++;
+        if (!(v <= thr)) continue;
+        pushed++;
+        const uint64_t key = make_key(v, idx);
+        lost = fminf(lost, key_d2(umax64(best, key)));  // (of no key yet: NaN, ignored)
+        if (key < best) {
+          best = key;
+          thr = fminf(thr, band_hi(v, a.d));
+          theta = sqrtf(thr);
+          slack = tol * (2.0f * D + 2.0f * theta);
+        }
+      }
+    }
+    const bool none = best == kKeyMax;
+    const float d2 = key_d2(best);
+    const int32_t base = a.qc_ref_base ? (int32_t)a.qc_ref_base[qc] : 0;
+    const bool defer = !none && !fp32_exact(a) && lost <= band_hi(d2, a.d);
+    // deferred: the band kernel settles the boundary; it reads the number of
+    // keys below the band and the k-th value from the last slot
+    a.out_idx[q] = defer ? 0 : (none ? -1 : key_idx(best) - base);
+    a.out_dist[q] = defer ? d2 : (none ? inf : (a.squared ? d2 : sqrtf(d2)));
+    if (defer) a.unres_slot[atomicAdd(a.unres_count, 1u)] = (int32_t)slot;
+  }
+  if (a.counters) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      evals += __shfl_xor_sync(kFull, evals, o);
+      visited += __shfl_xor_sync(kFull, visited, o);
+      pruned += __shfl_xor_sync(kFull, pruned, o);
+      pushed += __shfl_xor_sync(kFull, pushed, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&blk_ctr[0], (unsigned long long)evals);
+      atomicAdd(&blk_ctr[1], (unsigned long long)visited);
+      atomicAdd(&blk_ctr[2], (unsigned long long)pruned);
+      atomicAdd(&blk_ctr[3], (unsigned long long)pushed);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) atomicAdd(a.counters + threadIdx.x, blk_ctr[threadIdx.x]);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Band kernel: the k-th boundary of the queries the scan kernels could not
 // settle (a key of the final band was dropped for lack of room, or the
 // group scan's list holds one behind the k-th).  One block per query, over
@@ -2094,6 +2198,16 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
                      : a.d == 3 ? a.m_near >= a.n_ref
                      : a.d == 4 ? tiny || a.m_near >= (a.m >= 2 * fill ? 1 : 2) * a.n_ref
                                 : tiny || a.m_near >= 4 * a.n_ref;
+  // thread per query: the self-join's k = 1 in clusters of at most 128 points on
+  // average, from 8,192 queries on (5,000: d = 5 to 8 232 to 273 us by warps, 238
+  // to 252 by threads; 10,000, d = 8 371 and 285).  Other queries' nearest point
+  // is not in hand at once: 30,000 by 25,000 group 839 us, thread 1347.
+  if (a.k == 1 && a.qrows == a.rrows && a.d > 4 && a.dp4_tmpl == 2 && a.dorder &&
+      a.m >= 8192 && a.n_ref <= 128 * (int64_t)a.Rs) {
+    thread_scan_kernel<2><<<(unsigned)((a.m + 255) / 256), 256, 0, s>>>(a);
+    KNN_LAUNCH_CHECK();
+    return KNN_OK;
+  }
   if (a.k <= group_k && a.m >= fill && dense && a.slot_cl && (a.dp4_tmpl == 1 || a.dp4_tmpl == 2)) {
     if (a.dp4_tmpl == 1)
       return a.idx_in_row ? launch_group_scan<1, true>(a, num_sms, s)

@@ -140,8 +140,10 @@ int replicate_sides(Arena &ar, int g, int g0, const RefSide &R, const QuerySide 
     KNN_TRY(replicate(ar, g, g0, Q.order, (size_t)m, s, &order));
     Q2->order = order;
   }
-  if (R.boxes)
+  if (R.boxes) {
+    KNN_TRY(replicate(ar, g, g0, R.sset.perm, (size_t)n, s, &R2->sset.perm));
     KNN_TRY(replicate(ar, g, g0, Q.qset.reps, (size_t)Rq * dp4, s, &Q2->qset.reps));
+  }
   KNN_TRY(replicate(ar, g, g0, Q.qset.off, (size_t)Rq + 1, s, &Q2->qset.off));
   KNN_TRY(replicate(ar, g, g0, Q.slot_cl, (size_t)m, s, &Q2->slot_cl));
   KNN_TRY(replicate(ar, g, g0, Q.theta0, (size_t)Rq, s, &Q2->theta0));

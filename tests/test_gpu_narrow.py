@@ -112,3 +112,17 @@ def test_group_scan_limit_of_density(cuda_device, oracle, d, n, m):
     r = rng.uniform(-1, 1, (n, d)).astype(np.float32)
     q = rng.uniform(-1, 1, (m, d)).astype(np.float32)
     _check(oracle, q, r, 4, sample=150)
+
+
+@pytest.mark.parametrize("d", [5, 6, 7, 8])
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 9985])
+def test_thread_scan_selfjoin(cuda_device, oracle, d, n):
+    # k = 1 of a set with itself: copies of a point (the lowest row wins), rows on
+    # and off the integers, more than 128 points a cluster (not this kernel's)
+    rng = np.random.default_rng(100 * d + n)
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    x[n // 2:] = x[rng.integers(0, n // 2, n - n // 2)]
+    ints = rng.integers(0, 3, (n, d)).astype(np.float32)
+    for kw in ({}, {"sreps": n // 128 + 1, "qreps": n // 128 + 1}, {"sreps": 20, "qreps": 20}):
+        _check(oracle, x, x, 1, sample=200, **kw)
+        _check(oracle, ints, ints, 1, exact=True, sample=200, **kw)
