@@ -2185,18 +2185,17 @@ static int launch_scan_kernels(const ScanArgs &a, int num_sms, cudaStream_t s) {
   // box of 32 distant ones reaches blocks that none of them needs, the more so
   // the more dimensions there are.  Whole joins in us, group / warp, n reference
   // rows by m queries, uniform points unless said otherwise: d = 3, k = 16,
-  // 150,000 by 40,000 741 / 658 (mixtures 775 to 895 / 673 to 716); d = 4, k = 16,
-  // 100,000 by 50,000 1202 / 826, 60,000 by 60,000 1073 / 850, 150,000 by 150,000
-  // 1542 / 1751; k = 4, 60,000 by themselves d = 5 1350 / 844, d = 6 2296 / 1171,
+  // 150,000 by 40,000 741 / 658 (mixtures 775 to 895 / 673 to 716), 100,000 by 50,000
+  // 690 / 676, k = 4 558 / 621; d = 4, k = 16, 100,000 by 50,000 1202 / 826, 60,000
+  // by 60,000 1073 / 850, 150,000 by 150,000 1542 / 1751; k = 4, 60,000 by themselves d = 5 1350 / 844, d = 6 2296 / 1171,
   // d = 8 5592 / 2453 (200 mixtures 546 / 537); d = 8, k = 4, 20,000 by 200,000
   // 4817 / 5682 (8 mixtures 1388 / 2569); d = 6, k = 4, 64 clouds of 2,000 704
   // / 1017 (8 mixtures 380 / 618); d = 2, k = 4, 100,000 by 50,000 446 / 560.
   const int64_t fill = (int64_t)num_sms * 32 * (a.k == 1 ? 3 : 8);
   const int group_k = a.d <= 4 ? 32 : (a.d <= 6 ? 8 : 4);
   const bool tiny = a.n_ref <= 100 * (int64_t)a.Rs;  // clusters of a few blocks
-  const bool dense = a.d <= 2   ? 2 * a.m_near >= a.n_ref
-                     : a.d == 3 ? a.m_near >= a.n_ref
-                     : a.d == 4 ? tiny || a.m_near >= (a.m >= 2 * fill ? 1 : 2) * a.n_ref
+  const bool dense = a.d <= 3   ? 2 * a.m_near >= a.n_ref
+                     : a.d == 4 ? tiny || 4 * a.m_near >= (a.m >= 2 * fill ? 3 : 8) * a.n_ref
                                 : tiny || a.m_near >= 4 * a.n_ref;
   // thread per query: the self-join's k = 1 in clusters of at most 128 points on
   // average, from 8,192 queries on (5,000: d = 5 to 8 232 to 273 us by warps, 238

@@ -102,8 +102,8 @@ def test_small_join_self_and_missing_slots(cuda_device):
     assert idx[2].tolist() == [-1] * 6  # no distance from a NaN query is a number
 
 
-@pytest.mark.parametrize("d,n,m", [(3, MANY - 1, MANY), (3, MANY + 1, MANY), (4, 40_000, 76_000),
-                                   (4, 40_000, 75_000), (6, 9000, MANY), (6, 10_000, MANY),
+@pytest.mark.parametrize("d,n,m", [(3, 2 * MANY, MANY), (3, 2 * MANY + 1, MANY), (4, 60_000, 76_000),
+                                   (4, 60_000, 75_000), (6, 9000, MANY), (6, 10_000, MANY),
                                    (8, 9600, MANY)])
 def test_group_scan_limit_of_density(cuda_device, oracle, d, n, m):
     # enough queries for groups of 32, but as many reference rows on both sides of
