@@ -126,3 +126,16 @@ def test_thread_scan_selfjoin(cuda_device, oracle, d, n):
     for kw in ({}, {"sreps": n // 128 + 1, "qreps": n // 128 + 1}, {"sreps": 20, "qreps": 20}):
         _check(oracle, x, x, 1, sample=200, **kw)
         _check(oracle, ints, ints, 1, exact=True, sample=200, **kw)
+
+
+@pytest.mark.parametrize("d,k", [(1, 32), (2, 2), (2, 8), (2, 17), (2, 32), (3, 32), (6, 4)])
+def test_group_scan_cut_columns(cuda_device, oracle, d, k):
+    # every list and column overflows with equal distances again and again, within
+    # a cluster and between clusters; both in whole numbers and off them
+    rng = np.random.default_rng(10 * d + k)
+    r = rng.integers(0, 3, (9000, d)).astype(np.float32)
+    q = rng.integers(0, 3, (MANY, d)).astype(np.float32)
+    for sreps in (0, 9):
+        _check(oracle, q, r, k, exact=True, sample=150, sreps=sreps, qreps=sreps)
+    r[::2] += np.float32(1e-3)
+    _check(oracle, q + np.float32(0.3), r, k, sample=150)
