@@ -222,13 +222,13 @@ int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d,
   // nearest representative (BF16 tensor-core arg-min + exact FP32 distance to
   // the winner for d >= 16, FP32 CUDA cores otherwise), then one sort into
   // clusters
-  auto cluster = [&](const float4 *x, int64_t cnt, int dist_bits) -> int {
+  auto cluster = [&](const float4 *x, int64_t cnt, bool by_distance) -> int {
     if (tc_assign)
       KNN_TRY(launch_assign_tc(x, cnt, dp4s, d, cs->reps, R, tc_scratch, cl, dr, err, s));
     else
       KNN_TRY(launch_assign(x, cnt, dp4s, cs->reps, R, cl, dr, s));
     KNN_TRY(launch_cluster_sort(cl, dr, cnt, R, keys, vals, cs->skeys, cs->perm, temp,
-                                temp_bytes, s, dist_bits));
+                                temp_bytes, s, by_distance));
     return launch_cluster_offsets(cs->skeys, cnt, R, cs->off, s);
   };
   // Lloyd steps: the representatives move to their clusters' centroids (the
@@ -257,14 +257,14 @@ int build_clusters(Arena &keep, Arena &ar, const float4 *rows, int64_t n, int d,
     KNN_TRY(ar.alloc(&split, split_scratch_words(R)));
     KNN_CUDA_TRY(cudaMemsetAsync(split, 0, sizeof(uint64_t), s));
     for (int it = 0; it < lloyd_iters; it++) {
-      // (twelve bits of the distance tell the far members of a cluster)
-      KNN_TRY(cluster(x, cnt, 12));
-      KNN_TRY(launch_centroids(x, dp4s, cs->perm, cs->off, R, cs->reps, s));
+      // (the centroid step finds a cluster's farthest member itself)
+      KNN_TRY(cluster(x, cnt, false));
+      KNN_TRY(launch_centroids(x, dp4s, cs->perm, cs->skeys, cs->off, R, cs->reps, s));
       KNN_TRY(launch_split_clusters(x, dp4s, cs->perm, cs->off, cs->skeys, R, split,
                                     cs->reps, s));
     }
   }
-  KNN_TRY(cluster(rows, n, 32));
+  KNN_TRY(cluster(rows, n, true));
   return KNN_OK;
 }
 

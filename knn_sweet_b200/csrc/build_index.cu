@@ -233,22 +233,32 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Lloyd step: every representative moves to the centroid of its members.
-// One block per cluster; members are read in cluster order (perm) and summed
+// Lloyd step: every representative moves to the centroid of its members, and the
+// farthest of them to the cluster's last place, where the split looks for it (a
+// sort by distance as well, which only the split needed, took N = 400,000, d = 128
+// from 3.80 to 4.21 ms).  One block per cluster; members are read in cluster order (perm) and summed
 // with a fixed assignment of members to threads and a fixed tree, so the
 // result does not depend on scheduling.  Empty clusters keep their
 // representative.  (Representative refinement is not in the reference, which
 // keeps the best of its random draws, knnjoin.cu:125-154.)
 __global__ void __launch_bounds__(256)
-    centroid_kernel(const float4 *__restrict__ rows, int dp4, const int32_t *__restrict__ perm,
+    centroid_kernel(const float4 *__restrict__ rows, int dp4, int32_t *perm, uint64_t *skeys,
                     const int32_t *__restrict__ off, float4 *__restrict__ reps) {
   // G = pow2 >= dp4 lanes read one member row (one float4 each, coalesced);
   // 256 / G groups take every (256/G)-th member; the groups' partial sums are
   // added in group order, so the result does not depend on scheduling.
   __shared__ float4 red[256];
+  __shared__ uint64_t far_of[8];
   const int c = blockIdx.x, tid = threadIdx.x;
   const int a = off[c], b = off[c + 1];
   if (b == a) return;
+  // the farthest member, the last of equally far ones (distance bits, place)
+  uint64_t far = 0;
+  for (int p = a + tid; p < b; p += 256)
+    far = umax64(far, (skeys[p] << 32) | (uint32_t)p);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) far = umax64(far, __shfl_xor_sync(kFull, far, o));
+  if ((tid & 31) == 0) far_of[tid >> 5] = far;
   int G = 1;
   while (G < dp4 && G < 256) G <<= 1;
   const int groups = 256 / G, g = tid / G, col = tid % G;
@@ -279,11 +289,21 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
+  if (tid == 0) {  // (every member is read)
+    for (int w = 1; w < 8; w++) far = umax64(far, far_of[w]);
+    const int p = (int)(uint32_t)far;
+    const int32_t row = perm[p];
+    const uint64_t key = skeys[p];
+    perm[p] = perm[b - 1];
+    skeys[p] = skeys[b - 1];
+    perm[b - 1] = row;
+    skeys[b - 1] = key;
+  }
 }
 
-int launch_centroids(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off, int R,
-                     float4 *reps, cudaStream_t s) {
-  centroid_kernel<<<R, 256, 0, s>>>(rows, dp4, perm, off, reps);
+int launch_centroids(const float4 *rows, int dp4, int32_t *perm, uint64_t *skeys,
+                     const int32_t *off, int R, float4 *reps, cudaStream_t s) {
+  centroid_kernel<<<R, 256, 0, s>>>(rows, dp4, perm, skeys, off, reps);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }
@@ -1077,14 +1097,14 @@ int launch_chunk_slots(const int32_t *qorder, int64_t m, int first, int chunk_ro
 int launch_cluster_sort(const int32_t *cl, const float *dr, int64_t n, int R,
                         uint64_t *keys, int32_t *vals, uint64_t *skeys,
                         int32_t *perm, void *temp, size_t temp_bytes,
-                        cudaStream_t s, int dist_bits) {
+                        cudaStream_t s, bool by_distance) {
   if (n == 0) return KNN_OK;
   cluster_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(cl, dr, n, keys, vals);
   KNN_LAUNCH_CHECK();
   int end_bit = 32;
   while ((1LL << (end_bit - 32)) < (int64_t)R) end_bit++;
   KNN_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, skeys,
-                                               vals, perm, (int)n, 32 - dist_bits, end_bit, s));
+                                               vals, perm, (int)n, by_distance ? 0 : 32, end_bit, s));
   ++launch_counter();
   return KNN_OK;
 }

@@ -117,18 +117,19 @@ size_t cluster_sort_temp_bytes(int64_t n, int R);
 // hash of (seed, i), so that no period of the data is sampled in step.
 int launch_sample_rows(const float4 *rows, int dp4, int64_t stride, int64_t cnt, uint32_t seed,
                        float4 *out, cudaStream_t s);
-int launch_centroids(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off, int R,
-                     float4 *reps, cudaStream_t s);
+// Moves every cluster's farthest member to its last place in perm and skeys, and
+// its representative to the centroid of its members.
+int launch_centroids(const float4 *rows, int dp4, int32_t *perm, uint64_t *skeys,
+                     const int32_t *off, int R, float4 *reps, cudaStream_t s);
 size_t split_scratch_words(int R);
 int launch_split_clusters(const float4 *rows, int dp4, const int32_t *perm, const int32_t *off,
                           const uint64_t *skeys, int R, uint64_t *scratch, float4 *reps,
                           cudaStream_t s);
-// Sorts (cluster, distance) keys; dist_bits < 32 orders the distances by
-// their upper bits only.
+// Rows by (cluster, distance), or by cluster alone; equal ones in row order.
 int launch_cluster_sort(const int32_t *cl, const float *dr, int64_t n, int R,
                         uint64_t *keys, int32_t *vals, uint64_t *skeys,
                         int32_t *perm, void *temp, size_t temp_bytes,
-                        cudaStream_t s, int dist_bits = 32);
+                        cudaStream_t s, bool by_distance = true);
 size_t chunk_slots_temp_bytes(int64_t m, int nchunks);
 int launch_chunk_slots(const int32_t *qorder, int64_t m, int first, int chunk_rows, int nchunks,
                        uint32_t *keys, uint32_t *keys_out, int32_t *vals, int32_t *slots,
