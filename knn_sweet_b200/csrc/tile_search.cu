@@ -207,9 +207,11 @@ __device__ __forceinline__ void stage_tile(unsigned char *tile, const float *sc,
 // The same for member rows in column blocks: thread t takes row t % kTM and
 // (with NT = 2 kTM) every other 16-byte group of its columns, so that a warp
 // reads 512 contiguous bytes per chunk, stores 16-byte groups of consecutive
-// rows without bank conflicts and adds up its row's sums without shuffles.
+// rows without bank conflicts and adds up its row's sums without shuffles: eight
+// columns in a row, then groups of them in pairs, as the shuffles added them (one
+// running sum over its share of the columns would round up to five times as often).
 // pos: the row's position (negative: zeros).  The second half's sums go to
-// part[0..3 kTM) and are added by the caller's barrier (finish_sums).
+// part[0..3 kTM); the caller adds them behind its barrier.
 template <int NT>
 __device__ __forceinline__ void stage_members(unsigned char *tile, const float *sc, int KD, int d,
                                               int dp4, const float4 *__restrict__ srows,
@@ -232,6 +234,8 @@ __device__ __forceinline__ void stage_members(unsigned char *tile, const float *
         if (ch + 1 < dp4) c1[u] = row[(size_t)(ch + 1) * kColStride];
       }
     }
+    float pn = 0.0f, pe = 0.0f, pt = 0.0f;  // the round's first pair of groups
+    float qn = 0.0f, qe = 0.0f, qt = 0.0f;  // the pair at hand
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       const int g = g0 + u * H, k0 = g << 3;
@@ -239,6 +243,7 @@ __device__ __forceinline__ void stage_members(unsigned char *tile, const float *
       const float v[8] = {c0[u].x, c0[u].y, c0[u].z, c0[u].w,
                           c1[u].x, c1[u].y, c1[u].z, c1[u].w};
       __align__(16) __nv_bfloat16 b[8];
+      float gn = 0.0f, ge = 0.0f, gt = 0.0f;
 #pragma unroll
       for (int e = 0; e < 8; e++) {
         const int kk = k0 + e;
@@ -246,13 +251,23 @@ __device__ __forceinline__ void stage_members(unsigned char *tile, const float *
         b[e] = __float2bfloat16_rn(x);
         const float xr = __bfloat162float(b[e]);
         const float df = __fsub_rn(x, xr);
-        sn = __fmaf_rn(x, x, sn);
-        se = __fmaf_rn(df, df, se);
-        st = __fmaf_rn(xr, xr, st);
+        gn = __fmaf_rn(x, x, gn);
+        ge = __fmaf_rn(df, df, ge);
+        gt = __fmaf_rn(xr, xr, gt);
       }
       *reinterpret_cast<uint4 *>(tile + tc::tile_offset(r, k0, KD)) =
           *reinterpret_cast<const uint4 *>(b);
+      if (u == 2) {
+        pn = qn, pe = qe, pt = qt;
+        qn = qe = qt = 0.0f;
+      }
+      qn += gn;
+      qe += ge;
+      qt += gt;
     }
+    sn += pn + qn;
+    se += pe + qe;
+    st += pt + qt;
   }
   float *on = h == 0 ? o_n : part, *oe = h == 0 ? o_e : part + kTM,
         *ot = h == 0 ? o_t : part + 2 * kTM;
