@@ -115,9 +115,13 @@ typedef struct knn_stats {
   int32_t sreps_used;
   int32_t kernels_launched; /* device kernels this call enqueued (a radix sort
                                counts as one)                                 */
-  int32_t refine_fallbacks; /* BF16 form: queries whose kept candidates did
-                               not fit the re-ranking buffer and went to the
-                               FP32 scan instead                              */
+  int32_t refine_fallbacks; /* BF16 form: queries that went to the FP32 scan
+                               instead: their kept candidates did not fit the
+                               re-ranking buffer, or their tile of up to 128
+                               queries reached more members than it should
+                               stream.  Of such tiles the first to be met go, so
+                               that the number may differ from run to run (the
+                               results do not)                                */
   int32_t band_queries;     /* queries whose k-th boundary was settled by the
                                band kernel (a key of the band did not fit the
                                scan's candidate list)                         */
