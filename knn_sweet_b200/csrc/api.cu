@@ -522,15 +522,6 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   KNN_CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
   const int nclu = c1 - c0;
 
-  // wide rows and many queries: the query clusters that reach farthest first
-  const bool whole = slot0 == 0 && nslot == m;
-  int32_t *corder = nullptr, *cstart = nullptr;
-  if (whole && R.col_blocks && m >= kOrderedQueries) {
-    KNN_TRY(ar.alloc(&corder, (size_t)nclu));
-    KNN_TRY(ar.alloc(&cstart, (size_t)nclu));
-    KNN_TRY(launch_cluster_order(Q.rlen, Q.qset.off, nclu, corder, cstart, s));
-  }
-
   // BF16+refine form: tensor-core tiles over the same candidate lists; the
   // FP32 scan below then runs only for the queries the tiles hand back.
   int grid = 0, cap = 0, P = 0;
@@ -538,6 +529,28 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
   const bool tiles = o.precision == KNN_BF16_REFINE && tile_search_supported(d, k, o.margin) &&
                      tile_search_geometry(d, k, o.margin, num_sms, &grid, &cap, &P, &smem) ==
                          KNN_OK;
+  // host destination and a large result: scan in row chunks (each chunk's
+  // slots still in query-cluster order) and copy every finished chunk back
+  // while the next one runs.  About 16 MB of results per chunk, 8 to 32
+  // chunks (k = 200 self-join, 392 MB of results: 8.43 ms end to end with 8
+  // chunks, 8.18 with 24, 8.17 with 32; the copy alone takes 6.89 ms), the
+  // first one small (8.23 -> 8.10 ms on a box whose copy takes 7.15 ms)
+  const bool whole = slot0 == 0 && nslot == m;
+  const int64_t out_bytes = m * (int64_t)k * 8;
+  const int nchunks =
+      (sink && whole && !tiles && out_bytes >= (16 << 20) && m >= 8 * 1024)
+          ? (int)std::min<int64_t>(32, std::max<int64_t>(8, out_bytes >> 24))
+          : 1;
+
+  // wide rows and many queries: the query clusters that reach farthest first
+  // (chunks of rows are searched in their own order)
+  int32_t *corder = nullptr, *cstart = nullptr;
+  if (whole && nchunks == 1 && R.col_blocks && m >= kOrderedQueries) {
+    KNN_TRY(ar.alloc(&corder, (size_t)nclu));
+    KNN_TRY(ar.alloc(&cstart, (size_t)nclu));
+    KNN_TRY(launch_cluster_order(Q.rlen + c0, Q.qset.off + c0, nclu, corder, cstart, s));
+  }
+
   int32_t *fb_slots = nullptr;
   unsigned *fb_count = reinterpret_cast<unsigned *>(ctr + kCtrFallback);
   if (tiles) {
@@ -646,17 +659,6 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
     a.slot_list = fb_slots;
     a.slot_count = fb_count;
   }
-  // host destination and a large result: scan in row chunks (each chunk's
-  // slots still in query-cluster order) and copy every finished chunk back
-  // while the next one runs.  About 16 MB of results per chunk, 8 to 32
-  // chunks (k = 200 self-join, 392 MB of results: 8.43 ms end to end with 8
-  // chunks, 8.18 with 24, 8.17 with 32; the copy alone takes 6.89 ms), the
-  // first one small (8.23 -> 8.10 ms on a box whose copy takes 7.15 ms)
-  const int64_t out_bytes = m * (int64_t)k * 8;
-  const int nchunks =
-      (sink && whole && !tiles && out_bytes >= (16 << 20) && m >= 8 * 1024)
-          ? (int)std::min<int64_t>(32, std::max<int64_t>(8, out_bytes >> 24))
-          : 1;
   if (nchunks > 1) {
     // the first chunk one query per resident warp of the scan, so that the
     // copy-back starts after about one query's time; the rest in equal chunks
@@ -716,7 +718,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
       unsigned *count;
       KNN_TRY(ar.alloc(&order, (size_t)m));
       KNN_TRY(ar.alloc(&count, 1));
-      KNN_TRY(launch_slot_order(Q.slot_cl, Q.qset.off, cstart, m, order, count, s));
+      KNN_TRY(launch_slot_order(Q.slot_cl, Q.qset.off, cstart, c0, m, order, count, s));
       a.slot_list = order;
       a.slot_count = count;
       a.list_full = true;

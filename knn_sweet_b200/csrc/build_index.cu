@@ -862,13 +862,13 @@ __global__ void __launch_bounds__(1024)
 
 __global__ void slot_order_kernel(const int32_t *__restrict__ slot_cl,
                                   const int32_t *__restrict__ qoff,
-                                  const int32_t *__restrict__ cstart, int64_t m,
+                                  const int32_t *__restrict__ cstart, int c0, int64_t m,
                                   int32_t *__restrict__ order, unsigned *count) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *count = (unsigned)m;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m;
        p += (int64_t)gridDim.x * blockDim.x) {
     const int c = slot_cl[p];
-    order[cstart[c] + (p - qoff[c])] = (int32_t)p;
+    order[cstart[c - c0] + (p - qoff[c])] = (int32_t)p;
   }
 }
 
@@ -888,9 +888,9 @@ int launch_cluster_order(const int32_t *rlen, const int32_t *qoff, int Rq, int32
   return go(cluster_order_kernel<8>, 8);  // Rq <= 8192
 }
 
-int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t *cstart,
+int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t *cstart, int c0,
                       int64_t m, int32_t *order, unsigned *count, cudaStream_t s) {
-  slot_order_kernel<<<grid_for(m, 256), 256, 0, s>>>(slot_cl, qoff, cstart, m, order, count);
+  slot_order_kernel<<<grid_for(m, 256), 256, 0, s>>>(slot_cl, qoff, cstart, c0, m, order, count);
   KNN_LAUNCH_CHECK();
   return KNN_OK;
 }

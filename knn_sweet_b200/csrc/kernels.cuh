@@ -87,10 +87,11 @@ struct ScanArgs {
 };
 
 // The query clusters by the length of their candidate lists, longest first
-// (Rq <= KNN_MAX_REPS), and the slots in that order of their clusters.
+// (Rq <= KNN_MAX_REPS), and the slots in that order of their clusters, of which
+// the first is cluster c0 of slot_cl and qoff.
 int launch_cluster_order(const int32_t *rlen, const int32_t *qoff, int Rq, int32_t *corder,
                          int32_t *cstart, cudaStream_t s);
-int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t *cstart,
+int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t *cstart, int c0,
                       int64_t m, int32_t *order, unsigned *count, cudaStream_t s);
 int launch_pack_rows(const float *src, int64_t n, int d, int dp4, float4 *dst,
                      cudaStream_t s);

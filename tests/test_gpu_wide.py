@@ -149,3 +149,15 @@ def test_long_lists_left_to_a_block(cuda_device, oracle, k):
     assert_matches(idx[rows], dist[rows], oi, od)
     assert (idx >= 0).all()
     assert 0 < st.dist_evals <= st.pairs_total
+
+
+def test_chunked_host_join_orders_no_clusters(cuda_device):
+    # 8,192 queries by 256 results go back in eight chunks of rows: three launches
+    # each, three to make them, and no order of the clusters, which only a scan of
+    # all slots follows; one query less is one scan
+    rng = np.random.default_rng(2)
+    r = rng.standard_normal((9000, 9)).astype(np.float32)
+    q = rng.standard_normal((8192, 9)).astype(np.float32)
+    launches = {m: knnjoin(q[:m], r, 256, sreps=100, qreps=100, stats=True)[2].kernels_launched
+                for m in (8191, 8192)}
+    assert launches[8192] - launches[8191] == 3 + 8 * 3 - 3
