@@ -69,9 +69,8 @@ extern "C" {
 /*
  * Options.  Defaults (knn_default_options): qreps = sreps = 0 meaning
  * "choose from the set size" (about sqrt(n)*1.6, at most 4096, and one for a
- * join of at most 4,096 reference and 16,384 query rows with d <= 8, which is
- * not worth clusters; the reference
- * takes them from argv[4], argv[5]: knnjoin.cu:997-998), seed = 2015
+ * join of at most 4,096 reference and 16,384 query rows with d <= 8 (2,048
+ * queries for k > 512), which is not worth clusters; the reference takes them from argv[4], argv[5]: knnjoin.cu:997-998), seed = 2015
  * (knnjoin.cu:199, 226), rep_trials = 10 (knnjoin.cu:195), precision = FP32,
  * margin = 32, autotune = 1.
  */

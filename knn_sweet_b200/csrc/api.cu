@@ -437,7 +437,7 @@ int join_device_impl(const float *q, int64_t m, const float *r, int64_t n,
   unsigned long long *ctr;
   KNN_TRY(ar.alloc(&ctr, kCtrCount));
   KNN_CUDA_TRY(cudaMemsetAsync(ctr, 0, kCtrCount * sizeof(unsigned long long), s));
-  if (small_join_fits(m, n, d, o)) {
+  if (small_join_fits(m, n, d, k, o)) {
     KNN_TRY(small_join(q, m, r, n, d, k, out_idx, out_dist, o, ar, ctr, s,
                        st ? evs.ev[1] : nullptr));
     return finish_stats(1, 1, sink, ctr, s, evs, st);

@@ -182,7 +182,7 @@ int search_clusters(const RefSide &R, const QuerySide &Q, int64_t m, int32_t k, 
                     unsigned long long *ctr);
 // Small joins of narrow rows (small_join.cu): whether a join takes that path,
 // and the join itself; `built` (or null) is recorded between its stages.
-bool small_join_fits(int64_t m, int64_t n, int d, const knn_options &o);
+bool small_join_fits(int64_t m, int64_t n, int d, int k, const knn_options &o);
 int small_join(const float *q, int64_t m, const float *r, int64_t n, int d, int k,
                int32_t *out_idx, float *out_dist, const knn_options &o, Arena &ar,
                unsigned long long *ctr, cudaStream_t s, cudaEvent_t built);

@@ -207,10 +207,14 @@ __global__ void __launch_bounds__(kPrepThreads)
 
 // Whether a join takes this path: narrow rows, few of them, and no
 // representative count asked for (then the clusters are what the caller
-// wants to see in the statistics).
-bool small_join_fits(int64_t m, int64_t n, int d, const knn_options &o) {
-  return d <= 8 && n >= 1 && n <= kSmallRows && m <= kSmallQueries && o.qreps == 0 &&
-         o.sreps == 0;
+// wants to see in the statistics).  A warp with more than 512 results walks most
+// of the blocks of a separated set without a bound to begin with, and there are
+// half as many such warps: 4,096 rows of 10 distant groups, d = 8, k = 700, by
+// themselves 453 us clustered, 681 here, 16,384 queries 1211 and 1961, 2,000 383
+// and 450 (uniform rows 516 and 365); k = 500, 16,384 queries 1678 and 1648.
+bool small_join_fits(int64_t m, int64_t n, int d, int k, const knn_options &o) {
+  return d <= 8 && n >= 1 && n <= kSmallRows && m <= (k <= 512 ? kSmallQueries : 2048) &&
+         o.qreps == 0 && o.sreps == 0;
 }
 
 // The join, on device pointers; `ctr` (kCtrCount counters, zeroed).  ev(i)

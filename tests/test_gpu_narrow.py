@@ -139,3 +139,17 @@ def test_group_scan_cut_columns(cuda_device, oracle, d, k):
         _check(oracle, q, r, k, exact=True, sample=150, sreps=sreps, qreps=sreps)
     r[::2] += np.float32(1e-3)
     _check(oracle, q + np.float32(0.3), r, k, sample=150)
+
+
+@pytest.mark.parametrize("m,k,small", [(2049, 512, True), (2048, 513, True), (2049, 513, False),
+                                       (4096, 1000, False)])
+def test_small_join_limit_of_k(cuda_device, oracle, m, k, small):
+    # many results of few rows: one cluster, or the clustered join
+    rng = np.random.default_rng(k)
+    r = (rng.standard_normal((4096, 5)) + 30.0 * rng.integers(0, 5, (4096, 1))).astype(np.float32)
+    q = (rng.standard_normal((m, 5)) + 30.0 * rng.integers(0, 5, (m, 1))).astype(np.float32)
+    idx, dist, st = knnjoin(q, r, k, stats=True)
+    rows = rng.permutation(m)[:100]
+    oi, od = oracle.bruteforce_f64(q[rows], r, k)
+    assert_matches(idx[rows], dist[rows], oi, od)
+    assert (st.sreps_used == 1) == small
