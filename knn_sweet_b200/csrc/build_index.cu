@@ -318,7 +318,7 @@ int launch_centroids(const float4 *rows, int dp4, int32_t *perm, uint64_t *skeys
 // the next assignment splits the receiver.  A pair moves only when the
 // receiver's radius is more than twice the median radius and the donor holds
 // fewer points than the median cluster.  Deterministic: both orders break
-// ties by cluster id.  One block; R <= 8192.
+// ties by cluster id.  R <= 8192.
 // Block 0 sorts the clusters by size, block 1 by radius (widest first), eight
 // keys per thread in registers; the last of the two to finish moves the
 // representatives.  (One block sorting both in shared memory: 165 us at 8,192
@@ -900,8 +900,9 @@ int launch_slot_order(const int32_t *slot_cl, const int32_t *qoff, const int32_t
 // one GPU, src/knnjoin.cu:1103-1129): the cluster's query count times the
 // summed sizes of the bands it can scan, each taken for the cluster as a
 // whole (members s of a surviving reference cluster Rs with
-// |d(Rq,Rs) - d(s,Rs)| <= rq + theta0), plus one per query.  One warp per
-// query cluster.
+// |d(Rq,Rs) - d(s,Rs)| <= rq + theta0), plus one per query.  The scans of narrow
+// rows skip blocks by their boxes instead, for which the bands stand here too:
+// both grow with the reach of the cluster's bound.  One warp per query cluster.
 __global__ void cluster_work_kernel(const float *__restrict__ drr, int Rq, int Rs,
                                     const float *__restrict__ qrad,
                                     const float *__restrict__ theta0,

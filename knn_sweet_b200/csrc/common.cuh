@@ -214,35 +214,14 @@ __device__ __forceinline__ int nearest_of_quad(const float4 *__restrict__ row,
   return b;
 }
 
-// Warp-cooperative lower bound: first position p in [0, n) of the ascending
-// array a with a[p] >= v (n if none).  32-ary search: each round the lanes
-// sample 32 evenly spaced positions and a ballot brackets the answer, so a
-// list of a few thousand members needs two dependent loads instead of ~11.
-// Must be called by all 32 lanes with the same arguments.
-__device__ __forceinline__ int warp_lower_bound(const float *__restrict__ a,
-                                                int n, float v, int lane) {
-  int lo = 0, hi = n;  // answer in [lo, hi]
-  while (hi - lo > 32) {
-    int step = (hi - lo + 31) >> 5;
-    int p = lo + (lane + 1) * step - 1;
-    bool lt = (p < hi) && (a[p] < v);
-    unsigned b = __ballot_sync(kFull, lt);
-    int c = __popc(b);
-    int nlo = lo + c * step;
-    int nhi = lo + (c + 1) * step - 1;  // a[nhi] >= v if nhi < hi
-    lo = nlo;
-    hi = nhi < hi ? nhi : hi;
-  }
-  int p = lo + lane;
-  bool lt = (p < hi) && (a[p] < v);
-  return lo + __popc(__ballot_sync(kFull, lt));
-}
-
 // A start for a walk up a sorted array towards the first a[i] >= v: a
 // position lo with a[i] < v for every i < lo and that first element at most
-// 31 places further on.  The 32-ary search of warp_lower_bound without its
-// last level, which saves a dependent load round trip; the walk's own range
-// test skips the few elements below v.
+// 31 places further on.  32-ary search: each round the lanes sample 32 evenly
+// spaced positions and a ballot brackets the answer, so that a list of a few
+// thousand members needs one dependent load instead of some eleven; the level
+// that would find the element itself is left out (a load round trip less), as
+// the walk's own range test skips the few elements below v.  Called by all 32
+// lanes with the same arguments.
 __device__ __forceinline__ int warp_lower_bound_coarse(const float *__restrict__ a, int n,
                                                        float v, int lane) {
   int lo = 0, hi = n;

@@ -219,7 +219,7 @@ int cluster_side(const Plan &p, const SideBufs &b, const float *src, int64_t n, 
   return rc;
 }
 
-int reps_for(int64_t n) {  // same default as knn_join_device
+int reps_for(int64_t n) {  // knn_join_device's for joins it clusters
   double r = std::floor(1.6 * std::sqrt((double)n) + 0.5);
   return (int)(r < 1 ? 1 : (r > 4096 ? 4096 : r));
 }

@@ -11,9 +11,12 @@
 // skewed cluster size distribution does not leave devices idle.
 //
 // knn_join_sharded builds the reference index and the query side ONCE, on
-// the first listed device, then copies what the search reads (rows, member
-// lists, bounds, candidate lists: N (4 dp4 + 12) bytes and Rq Rs 4 bytes of
-// lists) to every other device with peer copies over NVLink.  Each device
+// the first listed device, then copies what the search reads to every other
+// device with peer copies over NVLink: reference rows in both orders, distances
+// and indices (N (32 dp4 + 8) bytes), queries, keys, order and clusters (M (16
+// dp4 + 16), or M 16 of a self-join), lists with their bounds (Rq Rs 8), and for
+// narrow rows the orders by distance and by block (4 bytes a row each) and the
+// boxes (32 dp4 bytes per 32 rows and cluster).  Each device
 // searches its range and stores its results directly into the first
 // device's result buffer through peer memory (plain stores from the scan
 // kernels, no multicast); where peer access is not available a device
