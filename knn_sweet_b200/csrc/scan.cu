@@ -43,7 +43,8 @@
 namespace knnsweet {
 
 // Shared part of the top-k variants: the append buffer, the admission
-// threshold and what the FP64 re-check of the k-th boundary needs.
+// threshold and what the FP64 re-check of the k-th boundary needs.  kShared: the
+// other warps of a block lower the threshold too.
 //
 // The neighbour set must be the one an FP64 join gives.  Keys are FP32
 // (d^2, index) words, which rank two points differently from FP64 only when
@@ -72,7 +73,7 @@ enum {
 };
 constexpr int kStatKeys = (kStatWords + 1) / 2;  // 64-bit words they take
 
-template <int kLostOff, int kStatOff>
+template <int kLostOff, int kStatOff, bool kShared>
 struct TopKBase {
   uint64_t *buf;  // append buffer (shared memory)
   int nbuf, nlist, k;
@@ -112,9 +113,12 @@ struct TopKBase {
   }
   // threshold once the k-th squared distance is T: the FP32 band above it
   __device__ __forceinline__ void set_band_threshold(float T, int d) {
-    // (a threshold from the block's other warps may lie lower)
-    thr_d2 = fminf(thr_d2, band_hi(T, d));
-    theta = sqrtf(thr_d2);
+    float W = band_hi(T, d);
+    // a threshold from the block's other warps may lie lower (elsewhere the test
+    // cost the k = 200 self-join spills: 3.71 -> 3.75 ms)
+    if constexpr (kShared) W = fminf(thr_d2, W);
+    thr_d2 = W;
+    theta = sqrtf(W);
   }
   // a dropped key's distance word (NaN from an empty key is ignored)
   __device__ __forceinline__ void note_lost(uint32_t d2bits, int lane) {
@@ -128,9 +132,9 @@ struct TopKBase {
 // Small k: the sorted list of the best keys lives in registers
 // (one key per lane), with the FP32 band of the k-th kept behind it as far as
 // the 32 slots allow.
-template <int E>
-struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3> {
-  using B = TopKBase<64 * E + 2, 64 * E + 3>;
+template <int E, bool kShared>
+struct RegTopK : TopKBase<64 * E + 2, 64 * E + 3, kShared> {
+  using B = TopKBase<64 * E + 2, 64 * E + 3, kShared>;
   using B::buf, B::nbuf, B::nlist, B::k, B::count, B::note_lost, B::set_band_threshold,
       B::reset_threshold, B::settle;
   static constexpr int L = 32 * E;
@@ -255,9 +259,9 @@ __device__ __forceinline__ void smem_bitonic_sort(uint64_t *s, int lane) {
 #define KNN_TOPK_EARLY 160
 #endif
 
-template <int LL>
-struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129> {
-  using B = TopKBase<2 * LL + 128, 2 * LL + 129>;
+template <int LL, bool kShared>
+struct SelectTopK : TopKBase<2 * LL + 128, 2 * LL + 129, kShared> {
+  using B = TopKBase<2 * LL + 128, 2 * LL + 129, kShared>;
   using B::buf, B::nbuf, B::nlist, B::k, B::count, B::note_lost, B::set_band_threshold,
       B::reset_threshold, B::settle;
   static constexpr int L = LL;          // final sort length (pow2 >= k)
@@ -704,8 +708,8 @@ struct QueryRow<0, IDXROW> {
 #define KNN_REG_TOPK_MAX_K 24
 #endif
 
-template <int L>
-using TopKFor = std::conditional_t<(L <= 32), RegTopK<L / 32>, SelectTopK<L>>;
+template <int L, bool kShared>
+using TopKFor = std::conditional_t<(L <= 32), RegTopK<L / 32, kShared>, SelectTopK<L, kShared>>;
 
 // Rows of more than 8 floats keep 4+ float4 of the query in registers: those
 // kernels get the lower occupancy target instead of spilling.
@@ -735,7 +739,7 @@ constexpr int kShareLists = 32;
 template <int DP4, bool IDXROW, int L, int WARPS, bool ONE, bool SPLIT>
 __global__ void __launch_bounds__(WARPS * 32, (scan_min_blocks<DP4, WARPS>()))
     scan_kernel(const ScanArgs a) {
-  using TK = TopKFor<L>;
+  using TK = TopKFor<L, SPLIT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int dp4 = DP4 > 0 ? DP4 : a.dp4;
@@ -1193,7 +1197,7 @@ constexpr int kSplitWaves = 4;
 
 template <int DP4, bool IDXROW, int L, int WARPS, bool ONE>
 static int launch_scan_t(const ScanArgs &a, int num_sms, cudaStream_t s) {
-  using TK = TopKFor<L>;
+  using TK = TopKFor<L, false>;
   constexpr bool kWideRows = DP4 == 0 || DP4 >= 4;
   const size_t smem = (size_t)WARPS * TK::kSmemKeys * sizeof(uint64_t) +
                       (DP4 > 0 ? 0 : (size_t)WARPS * a.dp4 * sizeof(float4));
