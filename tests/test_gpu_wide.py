@@ -137,17 +137,28 @@ def test_few_clusters_ties(cuda_device, oracle, sreps):
         assert_matches(idx, dist, oi, od, exact=True)
 
 
+def _few_far_queries(k):
+    # 100 queries in the middle of 60,000 rows reach all of their hundred clusters
+    # and more; 4,900 in small groups far away are done at once, and leave the
+    # warps idle in which the others are given up
+    rng = np.random.default_rng(k)
+    groups = 1000.0 * rng.standard_normal((40, 16)) + 5000.0
+    r = np.concatenate([rng.standard_normal((60_000, 16)),
+                        groups[rng.integers(0, 40, 2000)] + 0.01 * rng.standard_normal((2000, 16))])
+    q = np.concatenate([2 * rng.standard_normal((100, 16)),
+                        groups[rng.integers(0, 40, 4900)] + 0.01 * rng.standard_normal((4900, 16))])
+    return r.astype(np.float32), q[rng.permutation(5000)].astype(np.float32)
+
+
 @pytest.mark.parametrize("k", [10, 40])
 def test_long_lists_left_to_a_block(cuda_device, oracle, k):
-    # no cluster out of reach, 100 of them: the last queries go to a block each
-    rng = np.random.default_rng(k)
-    r = rng.standard_normal((60_000, 16)).astype(np.float32)
-    q = (2 * rng.standard_normal((6000, 16))).astype(np.float32)
-    idx, dist, st = knnjoin(q, r, k, sreps=100, qreps=8, stats=True)
-    rows = rng.permutation(6000)[:200]
+    r, q = _few_far_queries(k)
+    idx, dist, st = knnjoin(q, r, k, sreps=150, qreps=60, stats=True)
+    far = np.flatnonzero(np.abs(q).max(1) < 100)
+    rows = np.concatenate([far, np.random.default_rng(1).permutation(5000)[:200]])
     oi, od = oracle.bruteforce_f64(q[rows], r, k)
     assert_matches(idx[rows], dist[rows], oi, od)
-    assert (idx >= 0).all()
+    assert (idx >= 0).all() and len(far) == 100
     assert 0 < st.dist_evals <= st.pairs_total
 
 
