@@ -1354,7 +1354,9 @@ __device__ __noinline__ float cut_column(uint32_t *col, int C, int n, int want, 
     if (x <= top) put(w++, x);
     else lost = fminf(lost, key_d2(x));
   }
-  if (w == want) return lost;
+  // (w >= want: while the keys of the last cut are all here they are want, and
+  // once one has gone above the threshold nothing above *ceil is left)
+  if (w <= want) return lost;
   for (n = w;; n--) {
     uint64_t most = 0;
     int at = 0;
